@@ -494,4 +494,238 @@ __device__ __forceinline__ void ifft2_pass2(const float2 *buf, int h, int lane, 
   });
 }
 
+// ---------------------------------------------------------------------------
+// The same two-warp transform with its twiddles inside the butterflies (group
+// form of the FT convolution).  With z = w^(8 m) and zeta = w^(m + 32 d1) the
+// two DFT8 of pass 2 take the twiddles between the passes as powers of one
+// number per transform:
+//   U_{p1}[d1]           = sum_p2 Z_{p1 + 8 p2}[m] z^p2   e^(2 pi i p2 d1 / 8)
+//   y[m + 32 d1 + 256 d2] = sum_p1 U_{p1}[d1]      zeta^p1 e^(2 pi i p1 d2 / 8)
+// so the table of w^(m p) (16 KB read per item) and the separate products
+// by it and by the 64th roots go: a radix-2 butterfly with a twiddle is six
+// multiply-adds, 72 per DFT8 (a plain DFT8 and its products: 84).
+//
+// (re, im) -> (im, re): packed instructions take an operand with its halves
+// swapped, both negated or one broadcast at no cost (instruction counts of a
+// loop of each form); a negated half of a value that is not a constant costs a
+// move, so those products stay scalar.
+__device__ __forceinline__ float2 cswap(float2 a) { return make_float2(a.y, a.x); }
+__device__ __forceinline__ float2 f2_fma(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2_pack(a)), "l"(f2_pack(b)), "l"(f2_pack(c)));
+  return f2_unpack(r);
+}
+__device__ __forceinline__ float2 f2_mul(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_pack(a)), "l"(f2_pack(b)));
+  return f2_unpack(r);
+}
+// t + i d and t - i d, one packed operation each
+__device__ __forceinline__ void add_sub_i2(float2 t, float2 d, float2 &plus, float2 &minus) {
+  plus = f2_fma(cswap(d), make_float2(-1.f, 1.f), t);
+  minus = f2_fma(cswap(d), make_float2(1.f, -1.f), t);
+}
+// a b = (a.x b.x - a.y b.y, a.x b.y + a.y b.x): a multiply and a multiply-add, packed
+__device__ __forceinline__ float2 cmul2(float2 a, float2 b) {
+  return f2_fma(make_float2(a.x, a.x), b, f2_mul(make_float2(-a.y, a.y), cswap(b)));
+}
+
+struct TwistedTw {
+  float2 t4, t2, t1, t1p;  // z^4, z^2, z, z e^(2 pi i / 8)
+};
+
+// (a, b) <- (a + t b, -(a - t b)): the second output is one packed operation
+// from the first, with its sign turned
+__device__ __forceinline__ void bfly(float2 &a, float2 &b, float2 t) {
+  const float2 h = f2_fma(make_float2(t.x, t.x), b, a);
+  const float2 p = make_float2(fmaf(-t.y, b.y, h.x), fmaf(t.y, b.x, h.y));
+  b = f2_fma(make_float2(-2.f, -2.f), a, p);
+  a = p;
+}
+// the same with i t
+__device__ __forceinline__ void bfly_i(float2 &a, float2 &b, float2 t) { bfly(a, b, make_float2(-t.y, t.x)); }
+
+// the second output from the inputs instead: where the first output is much the
+// larger one (a signal's peak), its rounding does not reach the second
+__device__ __forceinline__ void bfly_direct(float2 &a, float2 &b, float2 t) {
+  const float2 h = f2_fma(make_float2(t.x, t.x), b, a);
+  const float2 n = f2_fma(make_float2(t.x, t.x), b, make_float2(-a.x, -a.y));
+  a = make_float2(fmaf(-t.y, b.y, h.x), fmaf(t.y, b.x, h.y));
+  b = make_float2(fmaf(-t.y, b.y, n.x), fmaf(t.y, b.x, n.y));
+}
+
+__host__ __device__ constexpr int rev3(int k) { return ((k & 1) << 2) | (k & 2) | ((k >> 2) & 1); }
+
+// x[i] -> (-1)^popcount(k) sum_i x[i] z^i e^(2 pi i i k / 8) at x[rev3(k)].
+// LAST: the transform's last stage, outputs not taken from one another (2 us of
+// 314 at 2^21 bins x 85 rows; in every stage: 31 us).
+template <bool LAST>
+__device__ __forceinline__ void twisted_dft8(float2 *x, const TwistedTw &t) {
+  bfly(x[0], x[4], t.t4);
+  bfly(x[1], x[5], t.t4);
+  bfly(x[2], x[6], t.t4);
+  bfly(x[3], x[7], t.t4);
+  bfly(x[0], x[2], t.t2);
+  bfly(x[1], x[3], t.t2);
+  bfly_i(x[4], x[6], t.t2);
+  bfly_i(x[5], x[7], t.t2);
+  if constexpr (LAST) {
+    bfly_direct(x[0], x[1], t.t1);
+    bfly_direct(x[2], x[3], make_float2(-t.t1.y, t.t1.x));
+    bfly_direct(x[4], x[5], t.t1p);
+    bfly_direct(x[6], x[7], make_float2(-t.t1p.y, t.t1p.x));
+  } else {
+    bfly(x[0], x[1], t.t1);
+    bfly_i(x[2], x[3], t.t1);
+    bfly(x[4], x[5], t.t1p);
+    bfly_i(x[6], x[7], t.t1p);
+  }
+}
+
+// Twiddles of pass 2 of thread tp (m = 16 h + (l & 15), g = l >> 4), as powers
+// of w.  First DFT8: z' = w^(8 m) (-1)^g, which puts the thread's own outputs
+// d1 = 4 g + r into slots r and the partner's into slots 4 + r of both lane groups.
+__device__ __forceinline__ TwistedTw twisted_first(const float2 *__restrict__ table, int m, int g) {
+  const int e = 8 * m + 1024 * g;
+  TwistedTw t;
+  t.t4 = __ldg(table + ((4 * e) & 2047));
+  t.t2 = __ldg(table + ((2 * e) & 2047));
+  t.t1 = __ldg(table + (e & 2047));
+  t.t1p = __ldg(table + ((e + 256) & 2047));
+  return t;
+}
+// Second DFT8, one set per slot r: zeta = w^(m + 128 g + 32 r).  The thread's
+// own p1 half comes first, so for g = 1 the halves are swapped (sum over p1 =
+// i + 4 mod 8): the outputs turn by zeta^4 (-1)^d2, which |y|^2 removes, and
+// the step from the first half to the second is zeta^-4.  The partner's slots
+// carry one more sign flip than the thread's own (slot 4 + r against r), hence
+// the minus.
+__device__ __forceinline__ TwistedTw twisted_second(const float2 *__restrict__ table, int m, int g, int r) {
+  const int e = m + 128 * g + 32 * r;
+  TwistedTw t;
+  const float2 d = __ldg(table + ((g ? -4 * e : 4 * e) & 2047));
+  t.t4 = make_float2(-d.x, -d.y);
+  t.t2 = __ldg(table + ((2 * e) & 2047));
+  t.t1 = __ldg(table + (e & 2047));
+  t.t1p = __ldg(table + ((e + 256) & 2047));
+  return t;
+}
+
+// bfly with the compile-time twiddle e^(2 pi i J / N), 0 <= J < N / 2 (scalar
+// multiply-adds take the constants as immediates, packed ones would hold them
+// in registers)
+template <int N, int J>
+__device__ __forceinline__ void bfly_const(float2 &a, float2 &b) {
+  if constexpr (J == 0) {
+    const float2 t = b;
+    b = csub(a, t);
+    a = cadd(a, t);
+  } else if constexpr (4 * J == N) {
+    const float2 t = a, d = b;
+    add_sub_i2(t, d, a, b);
+  } else {
+    constexpr float c = kCos<N, J>, s = kSin<N, J>;
+    const float2 p = make_float2(fmaf(-s, b.y, fmaf(c, b.x, a.x)), fmaf(s, b.x, fmaf(c, b.y, a.y)));
+    b = f2_fma(make_float2(-2.f, -2.f), a, p);
+    a = p;
+  }
+}
+
+// Pass 1: v[a] = S[64 a + p] and the template values T(a) = T[64 a + p] on
+// entry, +-Z_p[m] = +-sum_a S T e^(2 pi i a m / 32) at v[pos_z(m)] on exit;
+// the sign depends on m only, and the outputs of one m only meet each other,
+// so |y|^2 does not see it.  4 x 8 split, a = 8 n1 + n2, m = k1 + 4 k2: half
+// of the products are part of the first butterflies (a0 +- S T), the twiddles
+// e^(2 pi i n2 k1 / 32) part of the DFT8's.
+__host__ __device__ constexpr int pos_z(int m) { return 8 * (m % 4) + rev3(m / 4); }
+template <typename Tmpl>
+__device__ __forceinline__ void twisted_pass1(float2 *v, Tmpl T) {
+  sfor<8>([&](auto N2) {
+    constexpr int n2 = decltype(N2)::value;
+    float2 x0 = cmul2(v[n2], T(n2)), x1 = cmul2(v[n2 + 8], T(n2 + 8)), x2 = v[n2 + 16], x3 = v[n2 + 24];
+    bfly(x0, x2, T(n2 + 16));
+    bfly(x1, x3, T(n2 + 24));
+    v[n2] = cadd(x0, x1);
+    v[n2 + 16] = csub(x0, x1);
+    add_sub_i2(x2, x3, v[n2 + 8], v[n2 + 24]);
+  });
+  sfor<4>([&](auto K1) {
+    constexpr int k1 = decltype(K1)::value;
+    float2 *x = v + 8 * k1;
+    // in 32nds of a turn: z^4 = 4 k1, z^2 = 2 k1, z = k1, z e^(2 pi i / 8) = k1 + 4
+    sfor<4>([&](auto I) { bfly_const<32, 4 * k1>(x[decltype(I)::value], x[decltype(I)::value + 4]); });
+    sfor<2>([&](auto I) {
+      constexpr int i = decltype(I)::value;
+      bfly_const<32, 2 * k1>(x[i], x[i + 2]);
+      bfly_const<32, 2 * k1 + 8>(x[i + 4], x[i + 6]);
+    });
+    bfly_const<32, k1>(x[0], x[1]);
+    bfly_const<32, k1 + 8>(x[2], x[3]);
+    bfly_const<32, k1 + 4>(x[4], x[5]);
+    bfly_const<32, k1 + 12>(x[6], x[7]);
+  });
+}
+// into the pair buffer as 16-byte pairs
+__device__ __forceinline__ void twisted_store(const float2 *v, float2 *buf, int p) {
+  float4 *row = reinterpret_cast<float4 *>(buf + kEx2Pitch * p);
+  sfor<16>([&](auto M2) {
+    constexpr int m = 2 * decltype(M2)::value;
+    const float2 a = v[pos_z(m)], b = v[pos_z(m + 1)];
+    row[m >> 1] = make_float4(a.x, a.y, b.x, b.y);
+  });
+}
+
+// Pass 2: put(r, d2, |y[m + 32 (4 g + r) + 256 d2]|^2) for the thread's 32
+// outputs.  ``tw.issue(k, t)`` starts the load of a set of twiddles into t
+// (k = 0: the first DFT8, 1 + r: slot r of the second) and ``tw.wait(t)``
+// completes it; ``after_read`` runs once the pair buffer has been read.
+template <typename Tw, typename Hook, typename Put>
+__device__ __forceinline__ void twisted_pass2(const float2 *buf, const Tw &tw, int tp, Hook after_read, Put put) {
+  const int l = tp & 31, m = 16 * (tp >> 5) + (l & 15), g = l >> 4;
+  const float2 *col = buf + kEx2Pitch * 4 * g + m;
+  TwistedTw t, tn;
+  tw.issue(0, t);
+  float2 u[32];  // u[8 q + p2], then slot s of q at u[8 q + rev3(s)]
+  sfor<4>([&](auto Q) {
+    constexpr int q = decltype(Q)::value;
+    sfor<8>([&](auto P2) {
+      constexpr int p2 = decltype(P2)::value;
+      u[8 * q + p2] = col[kEx2Pitch * (q + 8 * p2)];
+    });
+  });
+  tw.wait(t);
+  after_read();
+  sfor<4>([&](auto Q) { twisted_dft8<false>(u + 8 * decltype(Q)::value, t); });
+  tw.issue(1, t);
+  sfor<4>([&](auto Q) {
+    constexpr int q = decltype(Q)::value;
+    sfor<4>([&](auto R) {
+      float2 &x = u[8 * q + rev3(4 + decltype(R)::value)];
+      x.x = __shfl_xor_sync(0xffffffffu, x.x, 16);
+      x.y = __shfl_xor_sync(0xffffffffu, x.y, 16);
+    });
+  });
+  tw.wait(t);
+  sfor<4>([&](auto R) {
+    constexpr int r = decltype(R)::value;
+    if constexpr (r < 3) tw.issue(2 + r, tn);
+    float2 x[8];
+    sfor<4>([&](auto Q) {
+      constexpr int q = decltype(Q)::value;
+      x[q] = u[8 * q + rev3(r)];
+      x[4 + q] = u[8 * q + rev3(4 + r)];
+    });
+    twisted_dft8<true>(x, t);
+    sfor<8>([&](auto D2) {
+      constexpr int d2 = decltype(D2)::value;
+      const float2 y = x[rev3(d2)];
+      put(R, D2, fmaf(y.x, y.x, y.y * y.y));
+    });
+    if constexpr (r < 3) {
+      tw.wait(tn);
+      t = tn;
+    }
+  });
+}
+
 }  // namespace fdas

@@ -87,14 +87,15 @@ struct FtcParams {
   const float2 *twiddle;
   int *status;
   long long timeout_ns;
-  int ctas_per_sm;        // persistent CTAs per SM (1 leaves room for harmonic summing)
+  int ctas_per_sm;        // 1: the pair form, half an SM (leaves room for harmonic summing); else the group form
   int variant = 0;        // FFT split: 0 default, 1 one warp per item (64 x 32), 2 a warp pair (32 x 64);
                           // 3 / 4: tensor-core DFT factors with split BF16 / FP16 operands
   const BatchTrial *trials = nullptr;  // batched search: tiles of all trials, FOPs per trial
   int n_trials = 0;
   long long tile_begin = 0;  // batched search: global index of the launch's first tile
-  int inject_stall = 0;      // test hook: each warp pair's first template copy is announced on its
-                             // barrier but not issued, so that wait runs out (nothing is in flight)
+  int inject_stall = 0;      // test hook: the first template copy (of each CTA, or of each warp pair in the
+                             // pair form) is announced on its barrier but not issued, so that wait runs
+                             // out (nothing is in flight)
   // forward transform of the tiles on the tensor cores (precision form):
   // items are tiles, read from `input` (n_bins spectrum values) and written
   // to `tiles_out` as complex spectra

@@ -212,8 +212,9 @@ __global__ void __launch_bounds__(256, 1) ftc_kernel(FtcParams p) {
 }
 
 // ---------------------------------------------------------------------------
-// Two-warp variant: one warp pair per (tile, template) item, 32 values per
-// thread (<= 128 registers, two CTAs of 4 pairs per SM).  The pair buffer
+// Pair form, one CTA of 4 pairs per SM: half an SM's registers, so that harmonic
+// summing fits beside it (one warp pair per (tile, template) item, 32 values per
+// thread, <= 128 registers).  The pair buffer
 // (16.9 KB) holds the TMA-prefetched template spectrum of the item, then the
 // pass-1 exchange; the next item's template is prefetched into it as soon as
 // both warps have read the exchange back.
@@ -327,6 +328,287 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Group form, the FT convolution wherever it has the SMs for itself: 8 warp
+// pairs per CTA, one CTA per SM, each pair with one tile of a group of
+// consecutive tiles, all of them on the same template row at about the same time.  The template rows pass through a ring of shared-memory slots,
+// one 16 KB TMA copy for all pairs of the CTA.  The pair's tile spectrum and
+// its twiddles stay in tensor memory over the rows, used as 128 words of
+// private storage per thread (32 lanes x 128 columns per warp): registers hold
+// one transform only, and neither passes through L1 / shared memory again.
+// Work: the steps (group, row) in row-major order are split evenly over the
+// grid, so every CTA has the same number of steps to within one whatever the
+// number of tiles.
+// Bound by the shared-memory pipe and the FMA pipe about alike (2^19 bins x 85
+// rows: 64% and 63% busy, ~600 wavefronts and ~550 FMA-pipe clocks per item of
+// ~880 clocks); the pair form below moves ~960 wavefronts and 680 clocks per
+// item.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 314 / 89 / 17.5 us
+// against 432 / 118 / 19.4 us of the pair form.  The same with 6 pairs and the
+// tile in registers (168 a thread) took 361 us, 4 pairs of two rows each 488 us;
+// the twiddle products all packed 336 us, all scalar 345 us.
+constexpr int kGroupPairs = 8;
+constexpr int kGroupRing = 5;  // what 227 KB hold beside eight pair buffers
+constexpr int kGroupSmem = (kGroupRing * 2 * kTile + kGroupPairs * kEx2Floats) * (int)sizeof(float);
+constexpr int kGroupTmemCols = 512;
+// columns of a thread's 128: tile spectrum, then the twiddle sets of pass 2
+constexpr int kTmTile = 0, kTmTw = 64;
+
+struct GroupRing {
+  uint64_t full[kGroupRing];  // copy landed
+  unsigned used[kGroupRing];  // pairs that have read the slot's row
+  unsigned issued[kGroupRing];
+  int abort;
+  uint32_t tmem;
+};
+
+// Wait for a slot.  After a timeout the CTA goes on without waiting (its FOP is
+// reported as timed out), so no thread leaves a barrier of the others open.
+__device__ __forceinline__ void group_wait(GroupRing &ring, int slot, uint32_t parity, const FtcParams &p) {
+  if (mbar_try_wait(&ring.full[slot], parity)) return;
+  volatile int *stop = &ring.abort;
+  if (*stop) return;
+  const uint64_t t0 = gtimer();
+  while (!mbar_try_wait(&ring.full[slot], parity)) {
+    if (*stop) return;
+    if ((long long)(gtimer() - t0) > p.timeout_ns) {
+      atomicOr(p.status, kStatusFtcTimeout);
+      *stop = 1;
+      return;
+    }
+  }
+}
+
+// Tensor memory as the thread's own storage (32x32b: one word per lane and
+// column).  A load's registers hold its values after tm_wait_ld on them.
+#define TM_OUT4(v, i) "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i + 1].x), "=f"(v[i + 1].y)
+#define TM_IO4(v, i) "+f"(v[i].x), "+f"(v[i].y), "+f"(v[i + 1].x), "+f"(v[i + 1].y)
+#define TM_IN4(v, i) "f"(v[i].x), "f"(v[i].y), "f"(v[i + 1].x), "f"(v[i + 1].y)
+#define TM_16(M, v, i) M(v, i), M(v, i + 2), M(v, i + 4), M(v, i + 6), M(v, i + 8), M(v, i + 10), M(v, i + 12), M(v, i + 14)
+__device__ __forceinline__ void tm_ld16(uint32_t addr, float2 *v) {  // 16 complex values
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : TM_16(TM_OUT4, v, 0)
+      : "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tm_st16(uint32_t addr, const float2 *v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};" ::TM_16(TM_IN4, v, 0),
+      "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tm_wait_ld16(float2 *v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : TM_16(TM_IO4, v, 0)::"memory");
+}
+__device__ __forceinline__ void tm_ld_tw(uint32_t addr, TwistedTw &t) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(t.t4.x), "=f"(t.t4.y), "=f"(t.t2.x), "=f"(t.t2.y), "=f"(t.t1.x), "=f"(t.t1.y), "=f"(t.t1p.x),
+                 "=f"(t.t1p.y)
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void tm_st_tw(uint32_t addr, const TwistedTw &t) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"f"(t.t4.x),
+               "f"(t.t4.y), "f"(t.t2.x), "f"(t.t2.y), "f"(t.t1.x), "f"(t.t1.y), "f"(t.t1p.x), "f"(t.t1p.y), "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+struct TmemTwiddles {
+  uint32_t base;
+  __device__ __forceinline__ void issue(int k, TwistedTw &t) const { tm_ld_tw(base + kTmTw + 8 * k, t); }
+  __device__ __forceinline__ void wait(TwistedTw &t) const {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(t.t4.x), "+f"(t.t4.y), "+f"(t.t2.x), "+f"(t.t2.y), "+f"(t.t1.x), "+f"(t.t1.y), "+f"(t.t1p.x),
+                   "+f"(t.t1p.y)::"memory");
+  }
+};
+
+template <bool BATCH>
+__global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) {
+  extern __shared__ float4 smem_f4[];
+  __shared__ GroupRing ring;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int pair = warp >> 1;
+  const int tp = threadIdx.x & 63;  // thread of the pair
+  const int m = 16 * (warp & 1) + (lane & 15), g = lane >> 4;
+  float *slots = reinterpret_cast<float *>(smem_f4);
+  float2 *buf = reinterpret_cast<float2 *>(slots + kGroupRing * 2 * kTile + pair * kEx2Floats);
+  const int n_groups = (p.n_tiles + kGroupPairs - 1) / kGroupPairs;
+  const long long n_steps = (long long)n_groups * p.n_rows;
+  const long long first_step = n_steps * blockIdx.x / gridDim.x;
+  const int steps = (int)(n_steps * (blockIdx.x + 1) / gridDim.x - first_step);
+  int group = (int)(first_step / p.n_rows);
+  int rr = (int)(first_step - (long long)group * p.n_rows);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kGroupRing; ++i) {
+      mbar_init(&ring.full[i], 1);
+      ring.used[i] = 0;
+      ring.issued[i] = 0;
+    }
+    ring.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = 0; i < kGroupRing && i < steps; ++i) {
+      if (i == 0 && p.inject_stall) {  // test hook: a copy that never comes
+        mbar_arrive_expect_tx(&ring.full[0], kTile * 8);
+        continue;
+      }
+      prefetch_template(slots + i * 2 * kTile, p.tmpl + (long long)(p.row_begin + (rr + i) % p.n_rows) * kTile,
+                        &ring.full[i]);
+      ring.issued[i] = 1;
+    }
+  }
+  __syncwarp();
+  auto load_tile = [&](int tile, float2 *v) {
+    const float2 *s = p.tiles + (long long)tile * kTile + tp;
+    sfor<32>([&](auto A) {
+      constexpr int a = decltype(A)::value;
+      v[a] = __ldg(s + 64 * a);
+    });
+  };
+  uint32_t tm;
+  {  // the first tile and the twiddles are on their way while tensor memory is set up
+    float2 v[32];
+    const int tile = group * kGroupPairs + pair;
+    load_tile(min(tile, p.n_tiles - 1), v);
+    const TwistedTw tws[5] = {twisted_first(p.twiddle, m, g), twisted_second(p.twiddle, m, g, 0),
+                              twisted_second(p.twiddle, m, g, 1), twisted_second(p.twiddle, m, g, 2),
+                              twisted_second(p.twiddle, m, g, 3)};
+    if (warp == 0) {
+      // registers keep any other CTA of this size off the SM, so the columns are free
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&ring.tmem)),
+                   "r"(kGroupTmemCols));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // a warp reaches the 32 lanes of its quadrant; the four warps of a quadrant
+    // take 128 columns each
+    tm = ring.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(128 * (warp >> 2));
+    sfor<5>([&](auto K) { tm_st_tw(tm + kTmTw + 8 * decltype(K)::value, tws[decltype(K)::value]); });
+    tm_st16(tm + kTmTile, v);
+    tm_st16(tm + kTmTile + 32, v + 16);
+    tm_wait_st();
+  }
+  const TmemTwiddles tw{tm};
+
+  bool active = false, fresh = true, inner = false;
+  int lo = 0, hi = 0;
+  unsigned long long dst = 0;  // of output c = 0 in the step's FOP row
+  unsigned long long row_bytes = 0;
+  TrialCursor cur;
+  if constexpr (BATCH) cur.next_begin = -1;
+  int slot = 0;
+  uint32_t parity = 0;
+  int ahead = (rr + kGroupRing) % p.n_rows;  // row of the step a slot is refilled for
+  for (int i = 0; i < steps; ++i) {
+    if (fresh) {  // first step or a new group: this pair's tile
+      const int tile = group * kGroupPairs + pair;
+      active = tile < p.n_tiles;
+      if (active) {
+        if (i > 0) {
+          float2 v[32];
+          load_tile(tile, v);
+          tm_st16(tm + kTmTile, v);
+          tm_st16(tm + kTmTile + 32, v + 16);
+          tm_wait_st();
+        }
+        if constexpr (BATCH) {
+          if (cur.next_begin < 0) cursor_start<BATCH>(p, tile, cur);
+          cursor_seek<BATCH>(p, tile, cur);
+        }
+        const FopTarget tg = fop_target<BATCH>(p, tile, p.row_begin, cur);
+        if constexpr (BATCH) row_bytes = 4ull * (unsigned long long)cur.stride;
+        else row_bytes = 4ull * (unsigned long long)p.fop_stride;
+        // output n = mb + c, c = 32 r + 256 d2 known at compile time: the
+        // discard (n >= O) and the row end become two limits on c
+        const int mb = m + 128 * g;
+        const long long first_bin = tg.base + mb;
+        const long long room = (long long)tg.n_bins - first_bin;
+        lo = p.overlap - mb;
+        hi = room < kTile ? (int)room : kTile;
+        // all but the last tiles of a row keep no output below 256 and every
+        // one from 512 on (at the usual overlaps)
+        inner = p.overlap >= 256 && p.overlap <= 512 && tg.base + kTile <= tg.n_bins;
+        dst = reinterpret_cast<unsigned long long>(tg.out) + 4ull * static_cast<unsigned long long>(first_bin) +
+              row_bytes * (unsigned long long)rr;
+      }
+      fresh = false;
+    }
+    // the last pair to have read a slot refills it with the row kGroupRing steps on
+    auto release = [&]() {
+      if (tp == 0) {
+        __threadfence_block();
+        if (atomicAdd(&ring.used[slot], 1u) == kGroupPairs - 1) {
+          ring.used[slot] = 0;
+          __threadfence_block();
+          if (i + kGroupRing < steps && !*reinterpret_cast<volatile int *>(&ring.abort)) {
+            ring.issued[slot] += 1;
+            prefetch_template(slots + slot * 2 * kTile, p.tmpl + (long long)(p.row_begin + ahead) * kTile,
+                              &ring.full[slot]);
+          }
+        }
+      }
+      __syncwarp();
+    };
+    if (active) {
+      float2 v[32];
+      tm_ld16(tm + kTmTile, v);
+      tm_ld16(tm + kTmTile + 32, v + 16);
+      group_wait(ring, slot, parity, p);
+      __syncwarp();
+      tm_wait_ld16(v);
+      tm_wait_ld16(v + 16);
+      const float2 *row = reinterpret_cast<const float2 *>(slots + slot * 2 * kTile) + tp;
+      twisted_pass1(v, [&](int a) { return row[64 * a]; });
+      pair_sync(pair);  // template row and the previous item's exchange read by both warps
+      twisted_store(v, buf, tp);
+      pair_sync(pair);  // exchange written
+      const unsigned long long out = dst;
+      if (inner) {
+        twisted_pass2(buf, tw, tp, release, [&](auto R, auto D2, float pw) {
+          constexpr int r = decltype(R)::value, d2 = decltype(D2)::value, c = 32 * r + 256 * d2;
+          if (d2 >= 2 || (d2 == 1 && c >= lo)) *reinterpret_cast<float *>(out + 4ull * c) = pw;
+        });
+      } else {
+        twisted_pass2(buf, tw, tp, release, [&](auto R, auto D2, float pw) {
+          constexpr int r = decltype(R)::value, d2 = decltype(D2)::value, c = 32 * r + 256 * d2;
+          if (c >= lo && c < hi) *reinterpret_cast<float *>(out + 4ull * c) = pw;
+        });
+      }
+      __syncwarp();
+    } else {
+      group_wait(ring, slot, parity, p);
+      pair_sync(pair);  // no tile in the last group: the slot is handed on
+      release();
+    }
+    if (++slot == kGroupRing) {
+      slot = 0;
+      parity ^= 1u;
+    }
+    if (++ahead == p.n_rows) ahead = 0;
+    dst += row_bytes;
+    if (++rr == p.n_rows) {
+      rr = 0;
+      ++group;
+      fresh = true;
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(ring.tmem), "r"(kGroupTmemCols));
+  }
+  // every copy that was issued has landed before the CTA ends (after a
+  // timeout: waited for, bounded)
+  if (threadIdx.x == 0 && ring.abort)
+    for (int i = 0; i < kGroupRing; ++i)
+      if (ring.issued[i] && !(i == 0 && p.inject_stall)) mbar_wait(&ring.full[i], (ring.issued[i] - 1) & 1u, kDrainNs);
+}
+
 // FP64 DFT of the time-domain taps -> float spectra scaled by 2^-11.
 __global__ void spectra_kernel(SpectraParams p) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -385,8 +667,9 @@ cudaError_t launch_tile_fft(const TileParams &p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// FFT variant of the FT convolution: the two-warp form (default) or the
-// one-warp form; FDAS_FTC_VARIANT=1warp selects the latter.
+// FFT variant of the FT convolution: the forms of two warps per item (default:
+// the group form, or the pair form where one CTA per SM shall leave room for
+// harmonic summing) or the one-warp form; FDAS_FTC_VARIANT=1warp selects the latter.
 static int ftc_variant() {
   static int v = -1;
   if (v < 0) {
@@ -408,14 +691,19 @@ cudaError_t launch_ftc(const FtcParams &p, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const long long ctas = (items + kWarpsPerCta - 1) / kWarpsPerCta;
     kern<<<(int)(ctas < n_sm ? ctas : n_sm), 256, smem, s>>>(p);
+  } else if (p.ctas_per_sm != 1) {
+    auto kern = p.trials ? ftcg_kernel<true> : ftcg_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
+    if (e != cudaSuccess) return e;
+    const long long steps = (long long)((p.n_tiles + kGroupPairs - 1) / kGroupPairs) * p.n_rows;
+    kern<<<(int)(steps < n_sm ? steps : n_sm), 64 * kGroupPairs, kGroupSmem, s>>>(p);
   } else {
     const int smem = (kPairsPerCta * kEx2Floats + kTw2Floats) * (int)sizeof(float);
     auto kern = p.trials ? ftc2_kernel<true> : ftc2_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const long long ctas = (items + kPairsPerCta - 1) / kPairsPerCta;
-    const long long per_sm = p.ctas_per_sm >= 1 && p.ctas_per_sm <= 2 ? p.ctas_per_sm : 2;
-    kern<<<(int)(ctas < per_sm * n_sm ? ctas : per_sm * n_sm), 256, smem, s>>>(p);
+    kern<<<(int)(ctas < n_sm ? ctas : n_sm), 256, smem, s>>>(p);
   }
   return cudaGetLastError();
 }
