@@ -87,11 +87,19 @@ struct EmitBuf {
 // HP_1 = FOP[t][f], HP_j = HP_{j-1} + FOP[trunc(t/j)][f/j] accumulated in FP32
 // in this order -- hsum.py:95-120 / hms_baseline.cl.mako:55-84 -- so the
 // values match hsum.py bit for bit for the same FOP.  A cell is a candidate of
-// plane j if HP_j > thr_j (strict, hsum.py:134 / detect.cl.mako:185).  The fast
-// path only tracks a bound of the tile maximum per plane and marks the planes
-// where some lane of the warp reaches the lower edge of the band; at the end
-// of the item, while the stage is still held, the warp recomputes its sums
-// plane by plane (same values, same order) and emits at the marked planes.
+// plane j if HP_j > thr_j (strict, hsum.py:134 / detect.cl.mako:185).
+//
+// The warps first look at upper bounds of the sums of their lanes' 4 x 4 cell
+// groups only; where no group's bound reaches a plane's band the item is done.
+// A few groups that do are summed one cell per lane (hs_few_groups); for more,
+// the warp sums its whole tile, marks the planes whose band some cell reaches,
+// and recomputes and emits at those (same values, same order).  The exact sums
+// of every cell cost 692 instructions per warp and item at about 5.6 clocks
+// each, and so held a stage for longer than its copies take; with the bounds
+// the copies set the pace.  Stage time (noise, with selection) at 2^21 bins x
+// 85 rows x 8 planes, 2^20 x 85 x 16, 300007 x 43 x 16, 2^15 x 85 x 8: 189 /
+// 166 / 70 / 30 us against 238 / 297 / 113 / 40; three strong signals at 2^21:
+// 253 against 292.
 struct HsItem {
   int f0, sgn, tlo;
 };
@@ -324,6 +332,270 @@ __device__ __noinline__ void hs_emit_item(const HsumParams *pp, const float *sta
   hs_emit_item_body<NW>(*pp, stage, eb, f0, sgn, tlo, t0, need);
 }
 
+// The exact sums of the warp's tile: planes (bit j - 1) where a cell of this
+// lane reaches the band.
+template <int MAXP, int NW>
+__device__ __forceinline__ unsigned hs_exact_marks(const HsumParams &p, const float *stage, int f0, int sgn, int tlo,
+                                                   int t0, int lane) {
+  // lane l holds bins f0 + 4 l + {0..3} and f0 + 128 + 4 l + {0..3}: the
+  // lanes of a warp read consecutive 16-byte words (no bank conflicts)
+  const int F = f0 + 4 * lane;
+  float acc[4][8];
+  hs_load_plane1<NW>(acc, stage, p, f0, sgn, tlo, t0, F);
+  // ub: an upper bound of the lane's tile maximum.  Rounded addition is
+  // monotone, so ub + (largest value added) bounds every new sum, and the
+  // exact maximum (a 3-input max tree) is only needed where the bound reaches
+  // a plane's band
+  float ub = max32(acc);
+  unsigned need_lane = ub >= p.trig[0] ? 1u : 0u;  // this lane's marks; one vote per item
+  hs_sfor<MAXP - 1>([&](auto JJ) {
+    constexpr int j = decltype(JJ)::value + 2;
+    if (j <= p.n_planes) {
+      const int a0 = (f0 / j) & ~3;
+      const int bw = p.bw[j], bh = p.bh[j];
+      const float *box = stage + p.soff[j];
+      // f0 is a multiple of 256, so for j = 2, 4, 8 the box starts at f0 / j
+      float vmax;
+      if constexpr (j == 2) {
+        const float *r0 = box + srow(t0 / 2, bh, sgn) * bw + 2 * lane;
+        const float *r1 = r0 + sgn * bw;
+        const float2 a0v = *reinterpret_cast<const float2 *>(r0), b0v = *reinterpret_cast<const float2 *>(r0 + 64);
+        const float2 a1v = *reinterpret_cast<const float2 *>(r1), b1v = *reinterpret_cast<const float2 *>(r1 + 64);
+        vmax = fmax3(fmax3(a0v.x, a0v.y, b0v.x), fmax3(b0v.y, a1v.x, a1v.y), fmaxf(b1v.x, b1v.y));
+  #pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const float2 va = kk < 2 ? a0v : a1v, vb = kk < 2 ? b0v : b1v;
+          add2(acc[kk][0], acc[kk][1], va.x, va.x);
+          add2(acc[kk][2], acc[kk][3], va.y, va.y);
+          add2(acc[kk][4], acc[kk][5], vb.x, vb.x);
+          add2(acc[kk][6], acc[kk][7], vb.y, vb.y);
+        }
+      } else if constexpr (j == 4) {
+        const float *r0 = box + srow(t0 / 4, bh, sgn) * bw + lane;
+        const float va = r0[0], vb = r0[32];
+        vmax = fmaxf(va, vb);
+  #pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+  #pragma unroll
+          for (int e = 0; e < 8; e += 2) add2(acc[kk][e], acc[kk][e + 1], e < 4 ? va : vb, e < 4 ? va : vb);
+      } else if constexpr (j == 8) {
+        const float *r0 = box + srow(t0 / 8, bh, sgn) * bw + (lane >> 1);
+        const float va = r0[0], vb = r0[16];
+        vmax = fmaxf(va, vb);
+  #pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+  #pragma unroll
+          for (int e = 0; e < 8; e += 2) add2(acc[kk][e], acc[kk][e + 1], e < 4 ? va : vb, e < 4 ? va : vb);
+      } else {
+        const int rb = t0 / j;
+        const int kstar = j - (t0 - rb * j);  // warp-uniform: first k with trunc((t0+k)/j) = rb + 1
+        const float *r0 = box + srow(rb, bh, sgn) * bw - a0;
+        const float *r1 = r0 + sgn * bw;
+        float c0[8], c1[8];
+        // bins F + c and F + 128 + c (c < 4) sit at (F + c) / j = qa + (ra + c >= j)
+        // (ra + 3 < 2 j), and likewise for the second group: two divisions per
+        // plane, and two staged values per group and row, qa and qa + 1
+        // (inside the box: bw >= 255 / j + 6)
+        const int qa = F / j, ra = F - qa * j;
+        const int qb = (F + 128) / j, rg = F + 128 - qb * j;
+        bool hi_a[4], hi_b[4];  // cell c takes the value at q + 1
+  #pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          hi_a[c] = ra + c >= j;
+          hi_b[c] = rg + c >= j;
+        }
+        const float2 va = make_float2(r0[qa], r0[qa + 1]), vb = make_float2(r0[qb], r0[qb + 1]);
+  #pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          c0[c] = hi_a[c] ? va.y : va.x;
+          c0[c + 4] = hi_b[c] ? vb.y : vb.x;
+        }
+        // the bound may include a value no cell takes: still an upper bound
+        vmax = fmaxf(fmaxf(va.x, va.y), fmaxf(vb.x, vb.y));
+        if (kstar < 4) {  // the second row only where the four rows split
+          const float2 wa = make_float2(r1[qa], r1[qa + 1]), wb = make_float2(r1[qb], r1[qb + 1]);
+  #pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            c1[c] = hi_a[c] ? wa.y : wa.x;
+            c1[c + 4] = hi_b[c] ? wb.y : wb.x;
+          }
+          vmax = fmax3(vmax, fmaxf(wa.x, wa.y), fmaxf(wb.x, wb.y));
+        } else {
+  #pragma unroll
+          for (int e = 0; e < 8; ++e) c1[e] = 0.f;
+        }
+        switch (kstar < 4 ? kstar : 4) {
+          case 1: add_rows<1>(acc, c0, c1); break;
+          case 2: add_rows<2>(acc, c0, c1); break;
+          case 3: add_rows<3>(acc, c0, c1); break;
+          default: add_rows<4>(acc, c0, c1); break;
+        }
+      }
+      ub += vmax;
+      if (ub >= p.trig[j - 1]) {  // per lane: no vote, no warp-wide branch in the plane loop
+        ub = max32(acc);
+        if (ub >= p.trig[j - 1]) need_lane |= 1u << (j - 1);
+      }
+    }
+  });
+  return need_lane;
+}
+
+// Where a warp's four rows lie in the staged box of plane j (float offset in
+// the stage of the first and the last of the rows trunc((t0 + k) / j); the rows
+// in between are one of the two), for both halves.
+template <int MAXP>
+struct HsRows {
+  unsigned pos[MAXP + 1] = {}, neg[MAXP + 1] = {};
+};
+template <int MAXP, int NW>
+__device__ __forceinline__ HsRows<MAXP> hs_rows(const HsumParams &p, int t0) {
+  HsRows<MAXP> r;
+  r.pos[1] = t0 * kHsBins;
+  r.neg[1] = (4 * NW - 4 - t0) * kHsBins;
+  hs_sfor<MAXP - 1>([&](auto JJ) {
+    constexpr int j = decltype(JJ)::value + 2;
+    if (j > p.n_planes) return;
+    const int a = t0 / j, b = (t0 + 3) / j, bw = p.bw[j], bh = p.bh[j], o = p.soff[j];
+    r.pos[j] = (unsigned)(o + a * bw) | (unsigned)(o + b * bw) << 16;
+    r.neg[j] = (unsigned)(o + (bh - 1 - a) * bw) | (unsigned)(o + (bh - 1 - b) * bw) << 16;
+  });
+  return r;
+}
+
+// Upper bounds of the sums in the lane's two 4 x 4 cell groups: per plane the
+// largest value any of a group's cells adds.  Rounded addition is monotone, so
+// a bound below a plane's band leaves no cell of the group in it -- which
+// settles 98% of the warps on noise at 8 planes with a third of the instructions
+// that every cell's own sums take.
+struct HsBounds {
+  float a, b;
+  bool hit_a, hit_b;
+};
+__device__ __forceinline__ float fmax4(float4 v) { return fmaxf(fmax3(v.x, v.y, v.z), v.w); }
+__device__ __forceinline__ void hs_bound_plane1(HsBounds &u, const float *stage, unsigned row, float trig, int lane) {
+  const float4 *r = reinterpret_cast<const float4 *>(stage + row) + lane;
+  const float4 a0 = r[0], a1 = r[kHsBins / 4], a2 = r[2 * (kHsBins / 4)], a3 = r[3 * (kHsBins / 4)];
+  const float4 b0 = r[32], b1 = r[kHsBins / 4 + 32], b2 = r[2 * (kHsBins / 4) + 32], b3 = r[3 * (kHsBins / 4) + 32];
+  u.a = fmaxf(fmax3(fmax4(a0), fmax4(a1), fmax4(a2)), fmax4(a3));
+  u.b = fmaxf(fmax3(fmax4(b0), fmax4(b1), fmax4(b2)), fmax4(b3));
+  u.hit_a = u.a >= trig;
+  u.hit_b = u.b >= trig;
+}
+// `where`: f0 mod j | (f0 / j - box start) << 8
+template <int j>
+__device__ __forceinline__ void hs_bound_plane(HsBounds &u, const float *stage, unsigned rows, int where, float trig,
+                                               int lane) {
+  const unsigned r0 = rows & 0xffffu, r1 = rows >> 16;
+  if constexpr (j == 2) {
+    const float2 *q0 = reinterpret_cast<const float2 *>(stage + r0) + lane;
+    const float2 *q1 = reinterpret_cast<const float2 *>(stage + r1) + lane;
+    const float2 a0 = q0[0], b0 = q0[32], a1 = q1[0], b1 = q1[32];
+    u.a += fmaxf(fmax3(a0.x, a0.y, a1.x), a1.y);
+    u.b += fmaxf(fmax3(b0.x, b0.y, b1.x), b1.y);
+  } else if constexpr (j == 4 || j == 8 || j == 16) {  // one value for the group
+    const float *q = stage + r0 + lane / (j / 4);
+    u.a += q[0];
+    u.b += q[128 / j];
+  } else {
+    // bins F .. F + 3 take at most two values, at F / j and (F + 3) / j; numbers
+    // below 300 divided by j <= 16 by a 16-bit reciprocal, exactly
+    constexpr unsigned M = 65536u / j + 1;
+    const unsigned x = (unsigned)(where & 0xff) + 4u * lane, o = (unsigned)where >> 8;
+    const unsigned qa = (x * M) >> 16, ha = ((x + 3) * M) >> 16;
+    const unsigned qb = ((x + 128) * M) >> 16, hb = ((x + 131) * M) >> 16;
+    const float *s0 = stage + r0 + o, *s1 = stage + r1 + o;
+    u.a += fmaxf(fmax3(s0[qa], s0[ha], s1[qa]), s1[ha]);
+    u.b += fmaxf(fmax3(s0[qb], s0[hb], s1[qb]), s1[hb]);
+  }
+  u.hit_a |= u.a >= trig;
+  u.hit_b |= u.b >= trig;
+}
+
+// The cells of a few 4 x 4 groups (bit l of hit_a / hit_b: lane l's group of
+// the first / second half of the bins), one cell per lane and two groups at a
+// time: their sums, and the hits and near-threshold cells among them.  On noise
+// a warp that does not pass on its bounds has one or two such groups, so this
+// is a fifth of the work of the whole tile's exact sums.
+constexpr int kHsFewGroups = 8;
+template <int MAXP, int NW>
+__device__ __forceinline__ void hs_few_groups_body(const HsumParams &p, const float *stage, EmitBuf *eb, int f0, int sgn,
+                                                   int tlo, int t0, unsigned hit_a, unsigned hit_b) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long todo = (unsigned long long)hit_b << 32 | hit_a;
+#pragma unroll 1
+  while (todo) {
+    int grp = __ffsll(todo) - 1;
+    todo &= todo - 1;
+    bool live = true;
+    if (lane >= 16) {  // the upper half-warp takes the next group, if there is one
+      live = todo != 0;
+      grp = live ? __ffsll(todo) - 1 : grp;
+    }
+    todo &= todo - 1;  // (0 stays 0)
+    const int t = t0 + ((lane >> 2) & 3), off = 4 * (grp & 31) + (grp & 32) * 4 + (lane & 3);
+    live = live && t <= p.half && t >= tlo && f0 + off < p.n_bins;
+    float hp[MAXP];
+    hp[0] = stage[p.soff[1] + srow(t, 4 * NW, sgn) * kHsBins + off];
+    hs_sfor<MAXP - 1>([&](auto JJ) {
+      constexpr int j = decltype(JJ)::value + 2;
+      if (j <= p.n_planes) {
+        const int a0 = (f0 / j) & ~3;
+        hp[j - 1] = stage[p.soff[j] + srow(t / j, p.bh[j], sgn) * p.bw[j] + (f0 + off) / j - a0];
+      }
+    });
+    unsigned hits = 0, near = 0;
+    hs_sfor<MAXP>([&](auto JJ) {
+      constexpr int i = decltype(JJ)::value;
+      if (i < p.n_planes) {
+        if constexpr (i > 0) hp[i] = hp[i - 1] + hp[i];
+        if (hp[i] > p.hi[i]) hits |= 1u << i;
+        else if (hp[i] >= p.lo[i]) near |= 1u << i;
+      }
+    });
+    if (!live) hits = near = 0;
+    if (__any_sync(0xffffffffu, hits | near)) {
+      const int row = p.half + sgn * t, bin = f0 + off;
+      const unsigned below = (1u << lane) - 1u;
+      hs_sfor<MAXP>([&](auto JJ) {
+        constexpr int i = decltype(JJ)::value;
+        if (i < p.n_planes) {
+          const unsigned mh = __ballot_sync(0xffffffffu, (hits >> i) & 1u);
+          if (mh) {
+            unsigned base = 0;
+            if (lane == 0) {
+              base = atomicAdd(p.cand_total, (unsigned)__popc(mh));
+              atomicAdd(&eb->pc[i], (unsigned)__popc(mh));
+              if (base + __popc(mh) > (unsigned)p.cand_cap) atomicOr(p.status, kStatusCandidateOverflow);
+            }
+            const unsigned g = __shfl_sync(0xffffffffu, base, 0) + __popc(mh & below);
+            if (((hits >> i) & 1u) && g < (unsigned)p.cand_cap) {
+              p.cand_key[g] = cand_key(i, row, bin);
+              p.cand_pwr[g] = hp[i];
+            }
+          }
+          const unsigned mn = __ballot_sync(0xffffffffu, (near >> i) & 1u);
+          if (mn) {
+            unsigned base = 0;
+            if (lane == 0) base = atomicAdd(p.rc_count, (unsigned)__popc(mn));
+            const unsigned g = __shfl_sync(0xffffffffu, base, 0) + __popc(mn & below);
+            if ((near >> i) & 1u) {
+              if (g < (unsigned)p.rc_cap) p.rc_list[g] = make_uint4((unsigned)i, (unsigned)row, (unsigned)bin, 0u);
+              else atomicOr(p.status, kStatusRecheckOverflow);
+            }
+          }
+        }
+      });
+    }
+  }
+}
+// (out of line where 16 consumer warps leave 96 registers: the caller's loop would spill)
+template <int MAXP, int NW>
+__device__ __noinline__ void hs_few_groups(const HsumParams *pp, const float *stage, EmitBuf *eb, int f0, int sgn,
+                                           int tlo, int t0, unsigned hit_a, unsigned hit_b) {
+  hs_few_groups_body<MAXP, NW>(*pp, stage, eb, f0, sgn, tlo, t0, hit_a, hit_b);
+}
+
 template <int MAXP, int NW, int kHsStages, int MINB>
 __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_constant__ HsumParams p,
                                                                     const __grid_constant__ HsumMaps m) {
@@ -334,8 +606,11 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
   uint64_t *full = reinterpret_cast<uint64_t *>(hs_smem);  // [kHsStages]
   uint64_t *full2 = full + kHsStages;                        // [kHsStages]
   uint64_t *empty = full2 + kHsStages;                       // [kHsStages]
-  int *item_id = reinterpret_cast<int *>(empty + kHsStages); // [kHsStages]
   HsumParams *sp = reinterpret_cast<HsumParams *>(hs_smem + 32);  // copy for the emitter
+  // per stage: [0] f0 of the item (-1: stop mark), [1] 2 tlo + (positive half),
+  // [j] f0 mod j | (f0 / j - start of the staged bins) << 8
+  int *item_at = reinterpret_cast<int *>(hs_smem + 200);  // [kHsStages][kItemWords]
+  constexpr int kItemWords = MAXP + 1;
   float *stages = hs_smem + 256;                             // 1 KB header
   EmitBuf &eb = *reinterpret_cast<EmitBuf *>(stages + kHsStages * p.stage_floats);
   constexpr int kRows1 = 4 * NW;
@@ -353,8 +628,8 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
     fence_mbar_init();
   }
   if (threadIdx.x < kMaxPlanes) eb.pc[threadIdx.x] = 0;
-  static_assert(sizeof(HsumParams) % 4 == 0 && 128 + sizeof(HsumParams) <= 1024, "header holds the parameters");
-  static_assert(kHsStages * (3 * 8 + 4) <= 128, "barriers and item ids before the parameter copy");
+  static_assert(sizeof(HsumParams) % 4 == 0 && 128 + sizeof(HsumParams) <= 800, "header holds the parameters");
+  static_assert(kHsStages * 3 * 8 <= 128 && 800 + kHsStages * kItemWords * 4 <= 1024, "barriers and items in the header");
   for (int i = threadIdx.x; i < (int)(sizeof(HsumParams) / 4); i += blockDim.x)
     reinterpret_cast<int *>(sp)[i] = reinterpret_cast<const int *>(&p)[i];
   __syncthreads();
@@ -391,7 +666,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
           // (a stage the test hook announced without copies has a phase that
           // never completes: no stop mark on it -- its consumers have left)
           if (drained && !(p.inject_stall && st == 0)) {
-            item_id[st] = -1;
+            item_at[st * kItemWords] = -1;
             mbar_arrive(full + st);
           }
           break;
@@ -406,11 +681,19 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
         }
         const int it = cur + used++;
         if (it >= n_items) {
-          item_id[st] = -1;
+          item_at[st * kItemWords] = -1;
           mbar_arrive(full + st);  // plain arrival: the stage carries the stop mark
           break;
         }
-        item_id[st] = it;
+        const HsItem item = hs_item(p, it);
+        int *at = item_at + st * kItemWords;
+        at[0] = item.f0;
+        at[1] = 2 * item.tlo + (item.sgn > 0);
+        hs_sfor<MAXP - 1>([&](auto JJ) {  // j known at compile time: divisions by constants
+          constexpr int j = decltype(JJ)::value + 2;
+          const int q = item.f0 / j;
+          at[j] = (item.f0 - q * j) | (q & 3) << 8;
+        });
         const unsigned bytes1 = (unsigned)(p.bw[1] * p.bh[1]) * 4u;
         if (p.inject_stall && s == 0) {  // test hook: announced, never issued -- nothing in flight
           mbar_arrive_expect_tx(full + st, bytes1);
@@ -420,7 +703,6 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
 #pragma unroll
         for (int q = 0; q < kHsStages; ++q)
           if (q == st) pending[q] = use;
-        const HsItem item = hs_item(p, it);
         float *stage = stages + st * p.stage_floats;
         mbar_arrive_expect_tx(full + st, bytes1);
         tma_load_2d(stage + p.soff[1], &m.map[1], item.f0, item.sgn > 0 ? H : H - (kRows1 - 1), full + st);
@@ -445,127 +727,42 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
   } else {
     // ------------------------------------------------------------ consumers
     const int t0 = 4 * warp;
+    const HsRows<MAXP> rows = hs_rows<MAXP, NW>(p, t0);
     for (int s = 0;; ++s) {
       const int st = s % kHsStages, use = s / kHsStages;
       if (!mbar_wait_parity(full + st, use & 1, p.timeout_ns)) {
         if (lane == 0) atomicOr(p.status, kStatusHsumTimeout);
         break;
       }
-      const int it = item_id[st];
-      if (it < 0) break;
-      const HsItem item = hs_item(p, it);
-      const int f0 = item.f0, sgn = item.sgn;
+      const int *at = item_at + st * kItemWords;
+      const int f0 = at[0];
+      if (f0 < 0) break;
+      const int sgn = (at[1] & 1) ? 1 : -1, tlo = at[1] >> 1;
       const float *stage = stages + st * p.stage_floats;
-      // lane l holds bins f0 + 4 l + {0..3} and f0 + 128 + 4 l + {0..3}: the
-      // lanes of a warp read consecutive 16-byte words (no bank conflicts)
-      const int F = f0 + 4 * lane;
-      float acc[4][8];
-      hs_load_plane1<NW>(acc, stage, p, f0, sgn, item.tlo, t0, F);
-      unsigned need = 0;  // planes (bit j - 1) where some lane reached the band; warp-uniform
-      // ub: an upper bound of the lane's tile maximum.  Rounded addition is
-      // monotone, so ub + (largest value added) bounds every new sum, and the
-      // exact maximum (a 3-input max tree) is only needed where the bound reaches
-      // a plane's band
-      float ub = max32(acc);
-      unsigned need_lane = ub >= p.trig[0] ? 1u : 0u;  // this lane's marks; one vote per item
+      HsBounds u;
+      hs_bound_plane1(u, stage, sgn > 0 ? rows.pos[1] : rows.neg[1], p.trig[0], lane);
       if (!mbar_wait_parity(full2 + st, use & 1, p.timeout_ns)) {
         if (lane == 0) atomicOr(p.status, kStatusHsumTimeout);
         break;
       }
       hs_sfor<MAXP - 1>([&](auto JJ) {
         constexpr int j = decltype(JJ)::value + 2;
-        if (j <= P) {
-          const int a0 = (f0 / j) & ~3;
-          const int bw = p.bw[j], bh = p.bh[j];
-          const float *box = stage + p.soff[j];
-          // f0 is a multiple of 256, so for j = 2, 4, 8 the box starts at f0 / j
-          float vmax;
-          if constexpr (j == 2) {
-            const float *r0 = box + srow(t0 / 2, bh, sgn) * bw + 2 * lane;
-            const float *r1 = r0 + sgn * bw;
-            const float2 a0v = *reinterpret_cast<const float2 *>(r0), b0v = *reinterpret_cast<const float2 *>(r0 + 64);
-            const float2 a1v = *reinterpret_cast<const float2 *>(r1), b1v = *reinterpret_cast<const float2 *>(r1 + 64);
-            vmax = fmax3(fmax3(a0v.x, a0v.y, b0v.x), fmax3(b0v.y, a1v.x, a1v.y), fmaxf(b1v.x, b1v.y));
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              const float2 va = kk < 2 ? a0v : a1v, vb = kk < 2 ? b0v : b1v;
-              add2(acc[kk][0], acc[kk][1], va.x, va.x);
-              add2(acc[kk][2], acc[kk][3], va.y, va.y);
-              add2(acc[kk][4], acc[kk][5], vb.x, vb.x);
-              add2(acc[kk][6], acc[kk][7], vb.y, vb.y);
-            }
-          } else if constexpr (j == 4) {
-            const float *r0 = box + srow(t0 / 4, bh, sgn) * bw + lane;
-            const float va = r0[0], vb = r0[32];
-            vmax = fmaxf(va, vb);
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-              for (int e = 0; e < 8; e += 2) add2(acc[kk][e], acc[kk][e + 1], e < 4 ? va : vb, e < 4 ? va : vb);
-          } else if constexpr (j == 8) {
-            const float *r0 = box + srow(t0 / 8, bh, sgn) * bw + (lane >> 1);
-            const float va = r0[0], vb = r0[16];
-            vmax = fmaxf(va, vb);
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-              for (int e = 0; e < 8; e += 2) add2(acc[kk][e], acc[kk][e + 1], e < 4 ? va : vb, e < 4 ? va : vb);
-          } else {
-            const int rb = t0 / j;
-            const int kstar = j - (t0 - rb * j);  // warp-uniform: first k with trunc((t0+k)/j) = rb + 1
-            const float *r0 = box + srow(rb, bh, sgn) * bw - a0;
-            const float *r1 = r0 + sgn * bw;
-            float c0[8], c1[8];
-            // bins F + c and F + 128 + c (c < 4) sit at (F + c) / j = qa + (ra + c >= j)
-            // (ra + 3 < 2 j), and likewise for the second group: two divisions per
-            // plane, and two staged values per group and row, qa and qa + 1
-            // (inside the box: bw >= 255 / j + 6)
-            const int qa = F / j, ra = F - qa * j;
-            const int qb = (F + 128) / j, rg = F + 128 - qb * j;
-            bool hi_a[4], hi_b[4];  // cell c takes the value at q + 1
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              hi_a[c] = ra + c >= j;
-              hi_b[c] = rg + c >= j;
-            }
-            const float2 va = make_float2(r0[qa], r0[qa + 1]), vb = make_float2(r0[qb], r0[qb + 1]);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              c0[c] = hi_a[c] ? va.y : va.x;
-              c0[c + 4] = hi_b[c] ? vb.y : vb.x;
-            }
-            // the bound may include a value no cell takes: still an upper bound
-            vmax = fmaxf(fmaxf(va.x, va.y), fmaxf(vb.x, vb.y));
-            if (kstar < 4) {  // the second row only where the four rows split
-              const float2 wa = make_float2(r1[qa], r1[qa + 1]), wb = make_float2(r1[qb], r1[qb + 1]);
-#pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                c1[c] = hi_a[c] ? wa.y : wa.x;
-                c1[c + 4] = hi_b[c] ? wb.y : wb.x;
-              }
-              vmax = fmax3(vmax, fmaxf(wa.x, wa.y), fmaxf(wb.x, wb.y));
-            } else {
-#pragma unroll
-              for (int e = 0; e < 8; ++e) c1[e] = 0.f;
-            }
-            switch (kstar < 4 ? kstar : 4) {
-              case 1: add_rows<1>(acc, c0, c1); break;
-              case 2: add_rows<2>(acc, c0, c1); break;
-              case 3: add_rows<3>(acc, c0, c1); break;
-              default: add_rows<4>(acc, c0, c1); break;
-            }
-          }
-          ub += vmax;
-          if (ub >= p.trig[j - 1]) {  // per lane: no vote, no warp-wide branch in the plane loop
-            ub = max32(acc);
-            if (ub >= p.trig[j - 1]) need_lane |= 1u << (j - 1);
+        if (j <= P)
+          hs_bound_plane<j>(u, stage, sgn > 0 ? rows.pos[j] : rows.neg[j], at[j], p.trig[j - 1], lane);
+      });
+      const unsigned hit_a = __ballot_sync(0xffffffffu, u.hit_a), hit_b = __ballot_sync(0xffffffffu, u.hit_b);
+      if (hit_a | hit_b) {
+        if (__popc(hit_a) + __popc(hit_b) <= kHsFewGroups) {
+          if constexpr (NW <= 11) hs_few_groups_body<MAXP, NW>(p, stage, &eb, f0, sgn, tlo, t0, hit_a, hit_b);
+          else hs_few_groups<MAXP, NW>(sp, stage, &eb, f0, sgn, tlo, t0, hit_a, hit_b);
+        } else {
+          const unsigned need =
+              __reduce_or_sync(0xffffffffu, hs_exact_marks<MAXP, NW>(p, stage, f0, sgn, tlo, t0, lane));
+          if (need) {
+            if constexpr (MINB >= 2) hs_emit_item_body<NW>(p, stage, &eb, f0, sgn, tlo, t0, need);
+            else hs_emit_item<NW>(sp, stage, &eb, f0, sgn, tlo, t0, need);
           }
         }
-      });
-      need = __reduce_or_sync(0xffffffffu, need_lane);
-      if (need) {
-        if constexpr (MINB >= 2) hs_emit_item_body<NW>(p, stage, &eb, f0, sgn, item.tlo, t0, need);
-        else hs_emit_item<NW>(sp, stage, &eb, f0, sgn, item.tlo, t0, need);
       }
 
       // release the stage to the producer
