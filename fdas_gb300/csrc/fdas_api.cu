@@ -200,9 +200,12 @@ void rows_of(const fdas_handle *h, fdas_fop_part w, int *row_begin, int *n_rows)
 }
 
 // ------------------------------------------------- harmonic-summing geometry
-// Box shapes of the per-item staging (see hsum_kernel): plane 1 is 128 bins x
+// Box shapes of the per-item staging (see hsum_kernel): plane 1 is kHsBins bins x
 // 4 NW rows, plane j >= 2 covers bins [(f0/j) & ~3, ...) of the rows
-// trunc(|t|/j), |t| < 4 NW, with one spare row and column for the 2 x 2 windows.
+// trunc(|t|/j), |t| < 4 NW.  Where j divides kHsBins a block's bins f0/j .. are
+// aligned and just kHsBins / j; else up to (f0 + kHsBins - 4) / j + 1, the last
+// value the kernel reads, for any of its blocks (the shift of f0/j against its
+// 4-aligned start repeats every 4 j blocks).
 void hsum_geometry(const fdas_handle *h, HsumParams &p) {
   const int nw = hsum_warps(h->H);
   p.bw[1] = kHsBins;
@@ -212,8 +215,12 @@ void hsum_geometry(const fdas_handle *h, HsumParams &p) {
   off += p.bw[1] * p.bh[1];
   unsigned bytes = (unsigned)(p.bw[1] * p.bh[1] * 4);
   for (int j = 2; j <= h->P; ++j) {
-    p.bw[j] = ((kHsBins - 1) / j + 6 + 3) & ~3;
-    p.bh[j] = (4 * nw - 1) / j + 2;
+    int width = kHsBins / j;
+    if (kHsBins % j)
+      for (int f0 = 0; f0 < 4 * j * kHsBins; f0 += kHsBins)
+        width = std::max(width, (f0 + kHsBins - 4) / j + 2 - ((f0 / j) & ~3));
+    p.bw[j] = (width + 3) & ~3;
+    p.bh[j] = (4 * nw - 1) / j + 1;
     off = (off + 31) & ~31;  // 128-byte aligned TMA destinations
     p.soff[j] = off;
     off += p.bw[j] * p.bh[j];
@@ -384,7 +391,7 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   }
   hsum_geometry(h, p);
   p.item_counter = S.d_ctrl + kCtrlItems;
-  p.lean = h->cfg.overlap && P <= 8 && hsum_warps(H) == 11 ? 1 : 0;
+  p.lean = h->cfg.overlap && P <= 8 && hsum_warps(H) <= 11 ? 1 : 0;
   p.inject_stall = (h->inject & FDAS_INJECT_HSUM_STALL) ? 1 : 0;
   p.cand_key = S.d_key;
   p.cand_pwr = S.d_pwr;

@@ -115,7 +115,7 @@ struct HsumParams {
   float trig[kMaxPlanes]; // fast-path trigger: a cell needs a closer look if HP >= trig
   float hi[kMaxPlanes];   // candidate if HP > hi
   float lo[kMaxPlanes];   // recheck if lo <= HP <= hi (lo = +inf: never)
-  // staging boxes: plane 1 is 128 bins x 4 NW rows; plane j >= 2 is bw[j] bins
+  // staging boxes: plane 1 is kHsBins bins x 4 NW rows; plane j >= 2 is bw[j] bins
   // (from (f0/j) rounded down to 4) x bh[j] rows (trunc(t/j) of the half)
   int bw[kMaxPlanes + 1];
   int bh[kMaxPlanes + 1];
@@ -133,7 +133,7 @@ struct HsumParams {
   int rc_cap;
   int *status;
   long long timeout_ns;   // bound on every wait
-  int lean;               // 1: 3 stages and <= 80 registers (shares an SM with the FT convolution)
+  int lean;               // 1: fewer stages and registers (shares an SM with the FT convolution)
   int inject_stall = 0;   // test hook: the first stage of every CTA is announced on its barriers
                           // but its copies are not issued, so the consumers' waits run out
 };

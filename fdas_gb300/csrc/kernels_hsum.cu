@@ -100,21 +100,29 @@ struct EmitBuf {
 // 85 rows x 8 planes, 2^20 x 85 x 16, 300007 x 43 x 16, 2^15 x 85 x 8: 189 /
 // 166 / 70 / 30 us against 238 / 297 / 113 / 40; three strong signals at 2^21:
 // 253 against 292.
+constexpr int kHsHeader = 1536;  // bytes before the stages: barriers, parameters, items
 struct HsItem {
   int f0, sgn, tlo;
 };
 
 __device__ __forceinline__ HsItem hs_item(const HsumParams &p, int it) {
-  // items enumerate (block, half) over the enabled halves, highest blocks
-  // first: a signal's harmonic images cover wider bin ranges at higher bins
-  // (plane j sums f/k for k <= j), so the items that emit most are handed
-  // out early and the light ones fill the end of the launch
+  // items enumerate (block, half) over the enabled halves.  Slots of the block
+  // order with o trailing one bits run down from the top of the lowest
+  // nb / 2^o blocks, so blocks b, b / 2, b / 4, ... are staged at about the
+  // same time and the sub-harmonic boxes of planes 2, 4, 8 (and 6 with 3) find
+  // the lower blocks in L2: at 2^21 bins 171 us a stage on noise and 244 with
+  // three strong signals, against 189 and 255 from the highest block down.
+  // Each octave starts with its highest blocks: a signal's harmonic images
+  // cover wider bin ranges at higher bins (plane j sums f/k for k <= j), so the
+  // items that emit most are handed out early and light ones end the launch.
   const bool neg = p.tlo[0] <= p.half, pos = p.tlo[1] <= p.half;
   const int nb = (p.n_bins + kHsBins - 1) / kHsBins;
-  int blk, halfsel;
-  if (neg && pos) { blk = it >> 1; halfsel = it & 1; }
-  else { blk = it; halfsel = pos ? 1 : 0; }
-  return HsItem{(nb - 1 - blk) * kHsBins, halfsel ? 1 : -1, p.tlo[halfsel]};
+  int slot, halfsel;
+  if (neg && pos) { slot = it >> 1; halfsel = it & 1; }
+  else { slot = it; halfsel = pos ? 1 : 0; }
+  const int o = __ffs(~slot) - 1;
+  const int blk = (nb >> o) - 1 - (slot >> (o + 1));
+  return HsItem{blk * kHsBins, halfsel ? 1 : -1, p.tlo[halfsel]};
 }
 
 __device__ __forceinline__ int hs_n_items(const HsumParams &p) {
@@ -395,7 +403,7 @@ __device__ __forceinline__ unsigned hs_exact_marks(const HsumParams &p, const fl
         // bins F + c and F + 128 + c (c < 4) sit at (F + c) / j = qa + (ra + c >= j)
         // (ra + 3 < 2 j), and likewise for the second group: two divisions per
         // plane, and two staged values per group and row, qa and qa + 1
-        // (inside the box: bw >= 255 / j + 6)
+        // (inside the box)
         const int qa = F / j, ra = F - qa * j;
         const int qb = (F + 128) / j, rg = F + 128 - qb * j;
         bool hi_a[4], hi_b[4];  // cell c takes the value at q + 1
@@ -441,26 +449,14 @@ __device__ __forceinline__ unsigned hs_exact_marks(const HsumParams &p, const fl
   return need_lane;
 }
 
-// Where a warp's four rows lie in the staged box of plane j (float offset in
-// the stage of the first and the last of the rows trunc((t0 + k) / j); the rows
-// in between are one of the two), for both halves.
-template <int MAXP>
-struct HsRows {
-  unsigned pos[MAXP + 1] = {}, neg[MAXP + 1] = {};
-};
-template <int MAXP, int NW>
-__device__ __forceinline__ HsRows<MAXP> hs_rows(const HsumParams &p, int t0) {
-  HsRows<MAXP> r;
-  r.pos[1] = t0 * kHsBins;
-  r.neg[1] = (4 * NW - 4 - t0) * kHsBins;
-  hs_sfor<MAXP - 1>([&](auto JJ) {
-    constexpr int j = decltype(JJ)::value + 2;
-    if (j > p.n_planes) return;
-    const int a = t0 / j, b = (t0 + 3) / j, bw = p.bw[j], bh = p.bh[j], o = p.soff[j];
-    r.pos[j] = (unsigned)(o + a * bw) | (unsigned)(o + b * bw) << 16;
-    r.neg[j] = (unsigned)(o + (bh - 1 - a) * bw) | (unsigned)(o + (bh - 1 - b) * bw) << 16;
-  });
-  return r;
+// Where a warp's four rows lie in the staged box of plane j: float offset in the
+// stage of the first row trunc(t0 / j) and, in the upper half-word, of the last,
+// trunc((t0 + 3) / j) (the rows in between are one of the two).
+template <int NW>
+__device__ __forceinline__ unsigned hs_row_offsets(const HsumParams &p, int j, int t0, int sgn) {
+  if (j == 1) return (unsigned)(sgn > 0 ? t0 : 4 * NW - 4 - t0) * kHsBins;
+  const int a = srow(t0 / j, p.bh[j], sgn), b = srow((t0 + 3) / j, p.bh[j], sgn);
+  return (unsigned)(p.soff[j] + a * p.bw[j]) | (unsigned)(p.soff[j] + b * p.bw[j]) << 16;
 }
 
 // Upper bounds of the sums in the lane's two 4 x 4 cell groups: per plane the
@@ -596,6 +592,11 @@ __device__ __noinline__ void hs_few_groups(const HsumParams *pp, const float *st
   hs_few_groups_body<MAXP, NW>(*pp, stage, eb, f0, sgn, tlo, t0, hit_a, hit_b);
 }
 
+// NW consumer warps cover the rows of a half, 4 each: 16 for banks above 87
+// rows, 11 above 47, else 6, whose stages are half as large so that five fit
+// (2^21 bins x 43 rows x 8 planes 133 us a stage against 155 with 11 warps and
+// 44-row boxes, 300007 x 43 x 16 64 against 71; a second group of 6 warps
+// taking every other stage changed neither).
 template <int MAXP, int NW, int kHsStages, int MINB>
 __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_constant__ HsumParams p,
                                                                     const __grid_constant__ HsumMaps m) {
@@ -611,8 +612,9 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
   // [j] f0 mod j | (f0 / j - start of the staged bins) << 8
   int *item_at = reinterpret_cast<int *>(hs_smem + 200);  // [kHsStages][kItemWords]
   constexpr int kItemWords = MAXP + 1;
-  float *stages = hs_smem + 256;                             // 1 KB header
+  float *stages = hs_smem + kHsHeader / 4;
   EmitBuf &eb = *reinterpret_cast<EmitBuf *>(stages + kHsStages * p.stage_floats);
+  unsigned *rows = reinterpret_cast<unsigned *>(&eb + 1);  // [NW][half][kMaxPlanes + 1]: hs_row_offsets
   constexpr int kRows1 = 4 * NW;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int H = p.half;
@@ -629,21 +631,32 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
   }
   if (threadIdx.x < kMaxPlanes) eb.pc[threadIdx.x] = 0;
   static_assert(sizeof(HsumParams) % 4 == 0 && 128 + sizeof(HsumParams) <= 800, "header holds the parameters");
-  static_assert(kHsStages * 3 * 8 <= 128 && 800 + kHsStages * kItemWords * 4 <= 1024, "barriers and items in the header");
+  static_assert(kHsStages * 3 * 8 <= 128 && 800 + kHsStages * kItemWords * 4 <= kHsHeader, "barriers and items in the header");
   for (int i = threadIdx.x; i < (int)(sizeof(HsumParams) / 4); i += blockDim.x)
     reinterpret_cast<int *>(sp)[i] = reinterpret_cast<const int *>(&p)[i];
+  for (int i = threadIdx.x; i < NW * 2 * (kMaxPlanes + 1); i += blockDim.x) {
+    const int j = i % (kMaxPlanes + 1), wh = i / (kMaxPlanes + 1);
+    rows[i] = j >= 1 && j <= P ? hs_row_offsets<NW>(p, j, 4 * (wh >> 1), wh & 1 ? 1 : -1) : 0u;
+  }
   __syncthreads();
 
   if (warp == NW) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
-      // items are taken from the global counter one at a time, the next one
-      // requested an item ahead so the atomic's latency is hidden (few items
-      // reserved per CTA keeps the end of the launch even)
-      constexpr int kChunk = 1;
-      int cur = (int)atomicAdd(p.item_counter, (unsigned)kChunk);
-      int nxt = (int)atomicAdd(p.item_counter, (unsigned)kChunk);
-      int used = 0;
+      // The first item is the CTA's own index, the others come from the global
+      // counter, requested ahead: two at a time (the halves of a block) while
+      // there are plenty, so that an atomic, which takes about as long as an
+      // item of a small bank, is out for two items; one at a time towards the
+      // end, which keeps it even.  2^21 bins x 43 rows: 134 us a stage against
+      // 147 one at a time; four at a time 131, but 263 against 245 where
+      // signals make neighbouring items slow (85 rows, three strong signals).
+      const int grid = gridDim.x;
+      int cur = blockIdx.x, cur_n = 1, used = 0;
+      auto request = [&](int seen, int &n) {
+        n = seen + 8 * grid < n_items ? 2 : 1;
+        return grid + (int)atomicAdd(p.item_counter, (unsigned)n);
+      };
+      int nxt_n, nxt = request(cur, nxt_n);
       // per stage: the use whose copies may still be in flight (-1: none).  A
       // stage's copies have landed once the consumers released it.
       int pending[kHsStages];
@@ -674,10 +687,11 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
 #pragma unroll
         for (int q = 0; q < kHsStages; ++q)
           if (q == st) pending[q] = -1;  // released by the consumers: its copies have landed
-        if (used == kChunk) {
+        if (used == cur_n) {
           cur = nxt;
+          cur_n = nxt_n;
           used = 0;
-          if (cur < n_items) nxt = (int)atomicAdd(p.item_counter, (unsigned)kChunk);
+          if (cur < n_items) nxt = request(cur, nxt_n);
         }
         const int it = cur + used++;
         if (it >= n_items) {
@@ -727,7 +741,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
   } else {
     // ------------------------------------------------------------ consumers
     const int t0 = 4 * warp;
-    const HsRows<MAXP> rows = hs_rows<MAXP, NW>(p, t0);
+    const unsigned *my_rows = rows + warp * 2 * (kMaxPlanes + 1);
     for (int s = 0;; ++s) {
       const int st = s % kHsStages, use = s / kHsStages;
       if (!mbar_wait_parity(full + st, use & 1, p.timeout_ns)) {
@@ -740,7 +754,8 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
       const int sgn = (at[1] & 1) ? 1 : -1, tlo = at[1] >> 1;
       const float *stage = stages + st * p.stage_floats;
       HsBounds u;
-      hs_bound_plane1(u, stage, sgn > 0 ? rows.pos[1] : rows.neg[1], p.trig[0], lane);
+      const unsigned *rj = my_rows + (sgn > 0 ? kMaxPlanes + 1 : 0);
+      hs_bound_plane1(u, stage, rj[1], p.trig[0], lane);
       if (!mbar_wait_parity(full2 + st, use & 1, p.timeout_ns)) {
         if (lane == 0) atomicOr(p.status, kStatusHsumTimeout);
         break;
@@ -748,7 +763,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
       hs_sfor<MAXP - 1>([&](auto JJ) {
         constexpr int j = decltype(JJ)::value + 2;
         if (j <= P)
-          hs_bound_plane<j>(u, stage, sgn > 0 ? rows.pos[j] : rows.neg[j], at[j], p.trig[j - 1], lane);
+          hs_bound_plane<j>(u, stage, rj[j], at[j], p.trig[j - 1], lane);
       });
       const unsigned hit_a = __ballot_sync(0xffffffffu, u.hit_a), hit_b = __ballot_sync(0xffffffffu, u.hit_b);
       if (hit_a | hit_b) {
@@ -1086,37 +1101,47 @@ __global__ void __launch_bounds__(1024) select_finalize_kernel(SelectParams p) {
 }
 
 // ----------------------------------------------------------------- launchers
-int hsum_warps(int half) { return (half + 1 + 3) / 4 <= 11 ? 11 : 16; }
+int hsum_warps(int half) {
+  const int w = (half + 1 + 3) / 4;
+  return w <= 6 ? 6 : w <= 11 ? 11 : 16;
+}
 static int hsum_stages(const HsumParams &p) {
-  return (p.lean || p.n_planes > 8 || hsum_warps(p.half) != 11) ? 2 : 3;
+  switch (hsum_warps(p.half)) {
+    case 6: return p.lean ? 3 : 5;
+    case 11: return p.lean ? 2 : 3;
+    default: return 2;
+  }
 }
 
 int hsum_smem_bytes(const HsumParams &p) {
-  return 1024 + hsum_stages(p) * p.stage_floats * 4 + (int)sizeof(EmitBuf);
+  return kHsHeader + hsum_stages(p) * p.stage_floats * 4 + (int)sizeof(EmitBuf) +
+         hsum_warps(p.half) * 2 * (kMaxPlanes + 1) * 4;
 }
 
 template <int MAXP, int NW, int STAGES, int MINB>
 static cudaError_t launch_hsum_t(const HsumParams &p, const HsumMaps &m, cudaStream_t s) {
   const int smem = hsum_smem_bytes(p);
-  cudaError_t e =
-      cudaFuncSetAttribute(hsum_kernel<MAXP, NW, STAGES, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  auto kern = hsum_kernel<MAXP, NW, STAGES, MINB>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const int n_sm = current_sm_count();
   const int items = (p.n_bins + kHsBins - 1) / kHsBins * 2;
-  hsum_kernel<MAXP, NW, STAGES, MINB><<<items < n_sm ? items : n_sm, 32 * (NW + 1), smem, s>>>(p, m);
+  kern<<<items < n_sm ? items : n_sm, 32 * (NW + 1), smem, s>>>(p, m);
   return cudaGetLastError();
 }
 
 cudaError_t launch_hsum(const HsumParams &p, const HsumMaps &m, cudaStream_t s) {
-  if (hsum_warps(p.half) == 11) {
-    if (p.n_planes <= 8) {
+  const bool few = p.n_planes <= 8;
+  switch (hsum_warps(p.half)) {
+    case 6:
+      if (p.lean) return launch_hsum_t<8, 6, 3, 2>(p, m, s);
+      return few ? launch_hsum_t<8, 6, 5, 1>(p, m, s) : launch_hsum_t<16, 6, 5, 1>(p, m, s);
+    case 11:
       // lean: 2 stages and a register budget that fits next to one FT-convolution CTA
       if (p.lean) return launch_hsum_t<8, 11, 2, 2>(p, m, s);
-      return launch_hsum_t<8, 11, 3, 1>(p, m, s);
-    }
-    return launch_hsum_t<16, 11, 2, 1>(p, m, s);
+      return few ? launch_hsum_t<8, 11, 3, 1>(p, m, s) : launch_hsum_t<16, 11, 3, 1>(p, m, s);
+    default: return launch_hsum_t<16, 16, 2, 1>(p, m, s);
   }
-  return launch_hsum_t<16, 16, 2, 1>(p, m, s);
 }
 
 cudaError_t launch_split_taps(double2 *taps, long long n, cudaStream_t s) {
