@@ -88,6 +88,7 @@ struct FtcParams {
   int *status;
   long long timeout_ns;
   int ctas_per_sm;        // 1: the pair form, half an SM (leaves room for harmonic summing); else the group form
+  int group_tiles = 8;    // group form: tiles per CTA and step (set by launch_ftc)
   int variant = 0;        // FFT split: 0 default, 1 one warp per item (64 x 32), 2 a warp pair (32 x 64);
                           // 3 / 4: tensor-core DFT factors with split BF16 / FP16 operands
   const BatchTrial *trials = nullptr;  // batched search: tiles of all trials, FOPs per trial

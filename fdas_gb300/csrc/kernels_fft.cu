@@ -434,8 +434,8 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
   const int m = 16 * (warp & 1) + (lane & 15), g = lane >> 4;
   float *slots = reinterpret_cast<float *>(smem_f4);
   float2 *buf = reinterpret_cast<float2 *>(slots + kGroupRing * 2 * kTile + pair * kEx2Floats);
-  const int n_groups = (p.n_tiles + kGroupPairs - 1) / kGroupPairs;
-  const long long n_steps = (long long)n_groups * p.n_rows;
+  const int gt = p.group_tiles;  // tiles of a group: the pairs that work
+  const long long n_steps = (long long)((p.n_tiles + gt - 1) / gt) * p.n_rows;
   const long long first_step = n_steps * blockIdx.x / gridDim.x;
   const int steps = (int)(n_steps * (blockIdx.x + 1) / gridDim.x - first_step);
   int group = (int)(first_step / p.n_rows);
@@ -470,8 +470,7 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
   uint32_t tm;
   {  // the first tile and the twiddles are on their way while tensor memory is set up
     float2 v[32];
-    const int tile = group * kGroupPairs + pair;
-    load_tile(min(tile, p.n_tiles - 1), v);
+    load_tile(min(group * gt + pair, p.n_tiles - 1), v);
     const TwistedTw tws[5] = {twisted_first(p.twiddle, m, g), twisted_second(p.twiddle, m, g, 0),
                               twisted_second(p.twiddle, m, g, 1), twisted_second(p.twiddle, m, g, 2),
                               twisted_second(p.twiddle, m, g, 3)};
@@ -503,9 +502,9 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
   int slot = 0;
   uint32_t parity = 0;
   int ahead = (rr + kGroupRing) % p.n_rows;  // row of the step a slot is refilled for
-  for (int i = 0; i < steps; ++i) {
+  for (int i = 0; i < (pair < gt ? steps : 0); ++i) {
     if (fresh) {  // first step or a new group: this pair's tile
-      const int tile = group * kGroupPairs + pair;
+      const int tile = group * gt + pair;
       active = tile < p.n_tiles;
       if (active) {
         if (i > 0) {
@@ -541,7 +540,7 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
     auto release = [&]() {
       if (tp == 0) {
         __threadfence_block();
-        if (atomicAdd(&ring.used[slot], 1u) == kGroupPairs - 1) {
+        if (atomicAdd(&ring.used[slot], 1u) == (unsigned)gt - 1u) {
           ring.used[slot] = 0;
           __threadfence_block();
           if (i + kGroupRing < steps && !*reinterpret_cast<volatile int *>(&ring.abort)) {
@@ -679,6 +678,27 @@ static int ftc_variant() {
   return v;
 }
 
+// Tiles per group of the group form: a step of 1 .. 8 tiles takes 1.24, 1.30,
+// 1.95, 2.00, 2.65, 2.70, 3.40, 3.45 us (slope over the rounds at 2^19 bins x 85
+// rows; an odd pair leaves two of the four schedulers a warp short), and the
+// launch as long as the CTA with the most steps.  Eight for long spectra (2^19:
+// 89 us, six 92, four 100); short ones do not fill their last round: 65536 bins
+// x 85 rows 22 us with six against 26 with eight, 2^17 33 against 35.
+static long long group_steps(int n_tiles, int n_rows, int gt) { return (long long)((n_tiles + gt - 1) / gt) * n_rows; }
+static int group_tiles(int n_tiles, int n_rows, int n_sm) {
+  static const int step_ns[kGroupPairs] = {1240, 1300, 1950, 2000, 2650, 2700, 3400, 3450};
+  int best = kGroupPairs;
+  long long best_ns = 0;
+  for (int gt = kGroupPairs; gt >= 1; --gt) {
+    const long long ns = (group_steps(n_tiles, n_rows, gt) + n_sm - 1) / n_sm * step_ns[gt - 1];
+    if (gt == kGroupPairs || ns < best_ns) {
+      best = gt;
+      best_ns = ns;
+    }
+  }
+  return best;
+}
+
 cudaError_t launch_ftc(const FtcParams &p, cudaStream_t s) {
   if (p.n_rows <= 0 || p.n_tiles <= 0) return cudaSuccess;
   const int n_sm = current_sm_count();
@@ -695,8 +715,10 @@ cudaError_t launch_ftc(const FtcParams &p, cudaStream_t s) {
     auto kern = p.trials ? ftcg_kernel<true> : ftcg_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
     if (e != cudaSuccess) return e;
-    const long long steps = (long long)((p.n_tiles + kGroupPairs - 1) / kGroupPairs) * p.n_rows;
-    kern<<<(int)(steps < n_sm ? steps : n_sm), 64 * kGroupPairs, kGroupSmem, s>>>(p);
+    FtcParams q = p;
+    q.group_tiles = group_tiles(p.n_tiles, p.n_rows, n_sm);
+    const long long steps = group_steps(p.n_tiles, p.n_rows, q.group_tiles);
+    kern<<<(int)(steps < n_sm ? steps : n_sm), 64 * kGroupPairs, kGroupSmem, s>>>(q);
   } else {
     const int smem = (kPairsPerCta * kEx2Floats + kTw2Floats) * (int)sizeof(float);
     auto kern = p.trials ? ftc2_kernel<true> : ftc2_kernel<false>;
