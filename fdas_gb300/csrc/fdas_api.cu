@@ -289,7 +289,21 @@ fdas_status enqueue_input(fdas_handle *h, int ab, const fdas_complex *input, boo
   return FDAS_OK;
 }
 
-fdas_status enqueue_tiling(fdas_handle *h, int ab) {
+// `chain`: the stages of one search are enqueued in one go (not a stage call, not
+// a capture).  The tiling then zeroes the control words for all of them, and
+// kernels may start on the tail of the one before (programmatic dependent launch).
+// Not where a later stage would be refused, whose call leaves the earlier
+// search's counts alone, nor for the tensor-core tiling, which zeroes nothing.
+bool can_chain(const fdas_handle *h, int ab, const float *thr) {
+  const BufferSet &S = h->set[ab];
+  HsumParams p{};
+  p.half = h->H;
+  p.n_planes = h->P;
+  hsum_geometry(h, p);
+  return !h->cfg.precision && S.have_templates && (thr || !S.thresholds.empty()) && hsum_smem_bytes(p) <= 227 * 1024;
+}
+
+fdas_status enqueue_tiling(fdas_handle *h, int ab, bool chain) {
   BufferSet &S = h->set[ab];
   TileParams p{};
   p.input = S.cur_input;
@@ -306,13 +320,17 @@ fdas_status enqueue_tiling(fdas_handle *h, int ab) {
                          h->wait_timeout_ns, S.stream));
     S.tile_unchecked = true;
   } else {
+    if (chain) {
+      p.zero = S.d_ctrl;
+      p.n_zero = kCtrlStride;
+    }
     CK(h, launch_tile_fft(p, S.stream));
   }
   CK(h, cudaEventRecord(S.ev[2], S.stream));
   return FDAS_OK;
 }
 
-fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which) {
+fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which, bool chain) {
   BufferSet &S = h->set[ab];
   if (!S.have_templates) return fail(h, FDAS_ERR_STATE, "templates not uploaded for this buffer set");
   if (!S.have_input) return fail(h, FDAS_ERR_STATE, "no input tiled on this buffer set");
@@ -346,8 +364,8 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which) {
   // two harmonic summings run side by side after both FT convolutions.
   if (S.input_from_host && !h->cfg.overlap && !h->cfg.sync_pipeline && h->set[1 - ab].ev_hsum_recorded)
     CK(h, cudaStreamWaitEvent(S.stream, h->set[1 - ab].ev_hsum, 0));
-  CK(h, cudaMemsetAsync(S.d_ctrl + kCtrlFtcStatus, 0, sizeof(unsigned), S.stream));
-  CK(h, launch_ftc(p, S.stream));
+  if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl + kCtrlFtcStatus, 0, sizeof(unsigned), S.stream));
+  CK(h, launch_ftc(p, S.stream, chain));
   CK(h, cudaEventRecord(S.ev[3], S.stream));
   S.ftc_unchecked = true;
   S.ev_ftc_recorded = true;
@@ -355,7 +373,7 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which) {
   return FDAS_OK;
 }
 
-fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_part which) {
+fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_part which, bool chain) {
   BufferSet &S = h->set[ab];
   const float *thr = thr_in;
   if (!thr) {
@@ -406,8 +424,8 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
 
   if (hsum_smem_bytes(p) > 227 * 1024)
     return fail(h, FDAS_ERR_UNSUPPORTED, "harmonic summing staging exceeds shared memory (too many templates x planes)");
-  CK(h, cudaMemsetAsync(S.d_ctrl, 0, sizeof(unsigned) * kCtrlWords, S.stream));
-  CK(h, launch_hsum(p, S.maps, S.stream));
+  if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl, 0, sizeof(unsigned) * kCtrlWords, S.stream));
+  CK(h, launch_hsum(p, S.maps, S.stream, chain));
   if (S.ev_hsum) {  // (the batched form's per-trial views have none)
     CK(h, cudaEventRecord(S.ev_hsum, S.stream));
     S.ev_hsum_recorded = true;
@@ -430,7 +448,7 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
     r.cand_count = S.d_ctrl + kCtrlCount;
     r.cand_cap = h->cap;
     r.status = p.status;
-    CK(h, launch_recheck(r, S.stream));
+    CK(h, launch_recheck(r, S.stream, chain));
   }
   SelectParams f{};
   f.cand_key = S.d_key;
@@ -451,7 +469,7 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   f.compat_pwr = S.d_cpwr;
   f.invalid_location = (uint32_t)((h->H + 1 + h->H) & 0x7f) << 22;  // encode(1, H+1, 0), gen_info.h:69
   f.status = p.status;
-  CK(h, launch_select(f, S.stream));
+  CK(h, launch_select(f, S.stream, chain));
   CK(h, cudaMemcpyAsync(S.h_ctrl, S.d_ctrl, sizeof(unsigned) * kCtrlStride, cudaMemcpyDeviceToHost, S.stream));
   CK(h, cudaEventRecord(S.ev[4], S.stream));
   S.ctrl_valid = true;
@@ -472,7 +490,7 @@ fdas_status release_pending(fdas_handle *h, int ab) {
   BufferSet &S = h->set[ab];
   if (!S.pending) return FDAS_OK;
   S.pending = false;
-  fdas_status st = enqueue_hsum(h, ab, S.p_thr.data(), S.p_which);
+  fdas_status st = enqueue_hsum(h, ab, S.p_thr.data(), S.p_which, false);
   if (st != FDAS_OK) return st;
   return enqueue_download(h, ab, S.p_loc, S.p_pwr);
 }
@@ -877,7 +895,7 @@ fdas_status fdas_perform_input_tiling(fdas_handle *h, const fdas_complex *input,
   CK(h, cudaSetDevice(h->cfg.device));
   fdas_status st = enqueue_input(h, ab, input, false);
   if (st != FDAS_OK) return st;
-  if ((st = enqueue_tiling(h, ab)) != FDAS_OK) return st;
+  if ((st = enqueue_tiling(h, ab, false)) != FDAS_OK) return st;
   if ((st = sync_set(h, ab)) != FDAS_OK) return st;
   logf(h, "[INFO] Preparation duration: %.3f ms", elapsed(h->set[ab].ev[1], h->set[ab].ev[2]));
   return FDAS_OK;
@@ -888,7 +906,7 @@ fdas_status fdas_perform_ft_convolution(fdas_handle *h, fdas_fop_part which, fda
   CHECK_SET(h, ab);
   if (!valid_part(which)) return fail(h, FDAS_ERR_INVALID_ARG, "invalid FOP part");
   CK(h, cudaSetDevice(h->cfg.device));
-  fdas_status st = enqueue_ftc(h, ab, which);
+  fdas_status st = enqueue_ftc(h, ab, which, false);
   if (st != FDAS_OK) return st;
   if ((st = sync_set(h, ab)) != FDAS_OK) return st;
   logf(h, "[INFO] FT convolution and IFFT duration: %.3f ms", elapsed(h->set[ab].ev[2], h->set[ab].ev[3]));
@@ -903,7 +921,7 @@ fdas_status fdas_perform_harmonic_summing(fdas_handle *h, const float *threshold
   CK(h, cudaSetDevice(h->cfg.device));
   BufferSet &S = h->set[ab];
   CK(h, cudaEventRecord(S.ev[3], S.stream));
-  fdas_status st = enqueue_hsum(h, ab, thresholds, which);
+  fdas_status st = enqueue_hsum(h, ab, thresholds, which, false);
   if (st != FDAS_OK) return st;
   if ((st = sync_set(h, ab)) != FDAS_OK) return st;
   logf(h, "[INFO] Harmonic summing duration: %.3f ms", elapsed(S.ev[3], S.ev[4]));
@@ -961,10 +979,12 @@ fdas_status fdas_launch(fdas_handle *h, const fdas_complex *input, const float *
   if (h->cfg.sync_pipeline && (st = release_pending(h, 1 - ab)) != FDAS_OK) return st;
   long long t[5];  // steady-clock times around the enqueue steps (FDAS.cpp:556-566)
   t[0] = steady_ns();
+  // (a held-back harmonic summing keeps the earlier search's results until it runs)
+  const bool chain = !h->cfg.sync_pipeline && can_chain(h, ab, thresholds);
   if ((st = enqueue_input(h, ab, input, false)) != FDAS_OK) return st;
-  if ((st = enqueue_tiling(h, ab)) != FDAS_OK) return st;
+  if ((st = enqueue_tiling(h, ab, chain)) != FDAS_OK) return st;
   t[1] = steady_ns();
-  if ((st = enqueue_ftc(h, ab, which)) != FDAS_OK) return st;
+  if ((st = enqueue_ftc(h, ab, which, chain)) != FDAS_OK) return st;
   t[2] = steady_ns();
   BufferSet &S = h->set[ab];
   if (h->cfg.sync_pipeline) {
@@ -977,7 +997,7 @@ fdas_status fdas_launch(fdas_handle *h, const fdas_complex *input, const float *
     S.launched = true;
     t[3] = t[4] = steady_ns();  // harmonic summing and download are enqueued later
   } else {
-    if ((st = enqueue_hsum(h, ab, thresholds, which)) != FDAS_OK) return st;
+    if ((st = enqueue_hsum(h, ab, thresholds, which, chain)) != FDAS_OK) return st;
     t[3] = steady_ns();
     if ((st = enqueue_download(h, ab, detection_location, detection_power)) != FDAS_OK) return st;
     t[4] = steady_ns();
@@ -1000,10 +1020,11 @@ fdas_status fdas_enqueue_search_device(fdas_handle *h, const fdas_complex *d_inp
   if (!valid_part(which)) return fail(h, FDAS_ERR_INVALID_ARG, "invalid FOP part");
   CK(h, cudaSetDevice(h->cfg.device));
   fdas_status st;
+  const bool chain = can_chain(h, ab, thresholds);
   if ((st = enqueue_input(h, ab, d_input, true)) != FDAS_OK) return st;
-  if ((st = enqueue_tiling(h, ab)) != FDAS_OK) return st;
-  if ((st = enqueue_ftc(h, ab, which)) != FDAS_OK) return st;
-  if ((st = enqueue_hsum(h, ab, thresholds, which)) != FDAS_OK) return st;
+  if ((st = enqueue_tiling(h, ab, chain)) != FDAS_OK) return st;
+  if ((st = enqueue_ftc(h, ab, which, chain)) != FDAS_OK) return st;
+  if ((st = enqueue_hsum(h, ab, thresholds, which, chain)) != FDAS_OK) return st;
   return enqueue_download(h, ab, nullptr, nullptr);
 }
 
@@ -1475,7 +1496,7 @@ fdas_status batch_enqueue(fdas_batch *b, const float *thr) {
     for (int i = i0; i < i1; ++i) {
       fdas_handle *v = b->views[i];
       v->cfg.overlap = (uint32_t)b->hsum_lean;  // the lean harmonic-summing kernel
-      fdas_status st = enqueue_hsum(v, 0, thr, FDAS_ALL_ACCELERATIONS);
+      fdas_status st = enqueue_hsum(v, 0, thr, FDAS_ALL_ACCELERATIONS, false);
       if (st != FDAS_OK) return bfail(b, st, v->err);
     }
     i0 = i1;

@@ -58,6 +58,7 @@ __global__ void noalloc_templates_kernel(const float2 *__restrict__ src, float2 
                                          int p4) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int r = blockIdx.y;
+  grid_release();
   if (k >= kTile || r >= n_templates) return;
   int q = k;
   if (p4) {
@@ -150,7 +151,10 @@ extern "C" fdas_status fdas_ft_convolution_noalloc(const fdas_complex *d_spectru
   tp.payload = (int)payload;
   tp.tiles = tiles;
   tp.twiddle = twiddle;
-  if (launch_tile_fft(tp, s) != cudaSuccess) {
+  // the kernels start on each other's tails; a capture gets plain launches
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool pdl = cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+  if (launch_tile_fft(tp, s, pdl) != cudaSuccess) {
     cudaGetLastError();
     return FDAS_ERR_CUDA;
   }
@@ -172,7 +176,7 @@ extern "C" fdas_status fdas_ft_convolution_noalloc(const fdas_complex *d_spectru
   fp.status = d_status ? reinterpret_cast<int *>(d_status) : status_word;
   fp.timeout_ns = 2000000000LL;  // 2 s
   fp.ctas_per_sm = 2;
-  if (launch_ftc(fp, s) != cudaSuccess) {
+  if (launch_ftc(fp, s, pdl) != cudaSuccess) {
     cudaGetLastError();
     return FDAS_ERR_CUDA;
   }

@@ -23,6 +23,11 @@ __global__ void __launch_bounds__(32 * kTileWarps, 3) tile_fft_kernel(TileParams
   extern __shared__ float4 smem_f4[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tile = blockIdx.x * kTileWarps + warp;
+  grid_release();
+  if (blockIdx.x == 0 && p.n_zero) {
+    grid_wait();
+    for (int i = threadIdx.x; i < p.n_zero; i += blockDim.x) p.zero[i] = 0u;
+  }
   if (tile >= p.n_tiles) return;
   float *ex = reinterpret_cast<float *>(smem_f4) + warp * kExFloats;
   const TwiddleBases tb = load_twiddle_bases<-1>(p.twiddle, lane);
@@ -37,6 +42,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 3) tile_fft_kernel(TileParams
     local = tile - tr.tile_begin;
   }
   const long long start = local * p.payload - p.overlap;
+  grid_wait();
   sfor<2>([&](auto C) {
     constexpr int c = decltype(C)::value;
     sfor<32>([&](auto D) {
@@ -441,6 +447,7 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
   int group = (int)(first_step / p.n_rows);
   int rr = (int)(first_step - (long long)group * p.n_rows);
 
+  grid_release();
   if (threadIdx.x == 0) {
     for (int i = 0; i < kGroupRing; ++i) {
       mbar_init(&ring.full[i], 1);
@@ -449,28 +456,18 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
     }
     ring.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int i = 0; i < kGroupRing && i < steps; ++i) {
-      if (i == 0 && p.inject_stall) {  // test hook: a copy that never comes
-        mbar_arrive_expect_tx(&ring.full[0], kTile * 8);
-        continue;
-      }
-      prefetch_template(slots + i * 2 * kTile, p.tmpl + (long long)(p.row_begin + (rr + i) % p.n_rows) * kTile,
-                        &ring.full[i]);
-      ring.issued[i] = 1;
-    }
   }
   __syncwarp();
+  // (past L1: each value is read once per group)
   auto load_tile = [&](int tile, float2 *v) {
     const float2 *s = p.tiles + (long long)tile * kTile + tp;
     sfor<32>([&](auto A) {
       constexpr int a = decltype(A)::value;
-      v[a] = __ldg(s + 64 * a);
+      v[a] = __ldcg(s + 64 * a);
     });
   };
   uint32_t tm;
-  {  // the first tile and the twiddles are on their way while tensor memory is set up
-    float2 v[32];
-    load_tile(min(group * gt + pair, p.n_tiles - 1), v);
+  {  // up to grid_wait nothing that the kernels before have written
     const TwistedTw tws[5] = {twisted_first(p.twiddle, m, g), twisted_second(p.twiddle, m, g, 0),
                               twisted_second(p.twiddle, m, g, 1), twisted_second(p.twiddle, m, g, 2),
                               twisted_second(p.twiddle, m, g, 3)};
@@ -480,6 +477,20 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
                    "r"(kGroupTmemCols));
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
+    grid_wait();
+    if (threadIdx.x == 0)
+      for (int i = 0; i < kGroupRing && i < steps; ++i) {
+        if (i == 0 && p.inject_stall) {  // test hook: a copy that never comes
+          mbar_arrive_expect_tx(&ring.full[0], kTile * 8);
+          continue;
+        }
+        prefetch_template(slots + i * 2 * kTile, p.tmpl + (long long)(p.row_begin + (rr + i) % p.n_rows) * kTile,
+                          &ring.full[i]);
+        ring.issued[i] = 1;
+      }
+    __syncwarp();
+    float2 v[32];
+    load_tile(min(group * gt + pair, p.n_tiles - 1), v);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -656,14 +667,13 @@ int current_sm_count() {
 
 static int ex_smem_bytes() { return kWarpsPerCta * kExFloats * (int)sizeof(float); }
 
-cudaError_t launch_tile_fft(const TileParams &p, cudaStream_t s) {
+cudaError_t launch_tile_fft(const TileParams &p, cudaStream_t s, bool pdl) {
   const int smem = kTileWarps * kExFloats * (int)sizeof(float);
   auto kern = p.trials ? tile_fft_kernel<true> : tile_fft_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   dim3 grid((p.n_tiles + kTileWarps - 1) / kTileWarps);
-  kern<<<grid, 32 * kTileWarps, smem, s>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(kern, grid, dim3(32 * kTileWarps), smem, s, pdl, p);
 }
 
 // FFT variant of the FT convolution: the forms of two warps per item (default:
@@ -699,7 +709,7 @@ static int group_tiles(int n_tiles, int n_rows, int n_sm) {
   return best;
 }
 
-cudaError_t launch_ftc(const FtcParams &p, cudaStream_t s) {
+cudaError_t launch_ftc(const FtcParams &p, cudaStream_t s, bool pdl) {
   if (p.n_rows <= 0 || p.n_tiles <= 0) return cudaSuccess;
   const int n_sm = current_sm_count();
   if ((p.variant == 3 || p.variant == 4) && !p.trials) return launch_ftc_tc(p, p.variant == 4, s);
@@ -718,7 +728,8 @@ cudaError_t launch_ftc(const FtcParams &p, cudaStream_t s) {
     FtcParams q = p;
     q.group_tiles = group_tiles(p.n_tiles, p.n_rows, n_sm);
     const long long steps = group_steps(p.n_tiles, p.n_rows, q.group_tiles);
-    kern<<<(int)(steps < n_sm ? steps : n_sm), 64 * kGroupPairs, kGroupSmem, s>>>(q);
+    return launch_kernel(kern, dim3((unsigned)(steps < n_sm ? steps : n_sm)), dim3(64 * kGroupPairs), kGroupSmem, s,
+                         pdl, q);
   } else {
     const int smem = (kPairsPerCta * kEx2Floats + kTw2Floats) * (int)sizeof(float);
     auto kern = p.trials ? ftc2_kernel<true> : ftc2_kernel<false>;

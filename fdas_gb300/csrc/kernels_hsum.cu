@@ -638,6 +638,8 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
     const int j = i % (kMaxPlanes + 1), wh = i / (kMaxPlanes + 1);
     rows[i] = j >= 1 && j <= P ? hs_row_offsets<NW>(p, j, 4 * (wh >> 1), wh & 1 ? 1 : -1) : 0u;
   }
+  grid_release();
+  grid_wait();
   __syncthreads();
 
   if (warp == NW) {
@@ -830,6 +832,8 @@ __global__ void __launch_bounds__(512) recheck_kernel(RecheckParams p) {
   __shared__ double cell[kMaxPlanes];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarps = blockDim.x >> 5;
+  grid_release();
+  grid_wait();
   const unsigned n = min(*p.rc_count, (unsigned)p.rc_cap);
   for (unsigned e = blockIdx.x; e < n; e += gridDim.x) {
     const uint4 ent = p.rc_list[e];
@@ -905,6 +909,8 @@ __global__ void __launch_bounds__(1024) select_hist_kernel(SelectParams p) {
   __shared__ bool over[kMaxPlanes];  // plane has more hits than K
   __shared__ int n_over;
   const int nb = p.n_planes * kSelBuckets;
+  grid_release();
+  grid_wait();
   if (threadIdx.x == 0) n_over = 0;
   __syncthreads();
   if (threadIdx.x < kMaxPlanes) {
@@ -991,6 +997,8 @@ __global__ void __launch_bounds__(1024) select_hist_kernel(SelectParams p) {
 
 __global__ void __launch_bounds__(256) select_gather_kernel(SelectParams p) {
   __shared__ int sb_of[kMaxPlanes];
+  grid_release();
+  grid_wait();
   if (threadIdx.x < kMaxPlanes) sb_of[threadIdx.x] = threadIdx.x < p.n_planes ? p.sel_bucket[threadIdx.x] : -1;
   __syncthreads();
   const unsigned n = min(*p.cand_total, (unsigned)p.cand_cap);
@@ -1039,6 +1047,7 @@ __device__ __forceinline__ bool stronger(float pa, unsigned long long ka, float 
 
 __global__ void __launch_bounds__(1024) select_finalize_kernel(SelectParams p) {
   extern __shared__ __align__(16) unsigned char fz_smem[];
+  grid_wait();
   const int plane = blockIdx.x;
   const int K = p.per_plane;
   unsigned long long *bkey = reinterpret_cast<unsigned long long *>(fz_smem);  // [kSortCap] boundary
@@ -1119,28 +1128,27 @@ int hsum_smem_bytes(const HsumParams &p) {
 }
 
 template <int MAXP, int NW, int STAGES, int MINB>
-static cudaError_t launch_hsum_t(const HsumParams &p, const HsumMaps &m, cudaStream_t s) {
+static cudaError_t launch_hsum_t(const HsumParams &p, const HsumMaps &m, cudaStream_t s, bool pdl) {
   const int smem = hsum_smem_bytes(p);
   auto kern = hsum_kernel<MAXP, NW, STAGES, MINB>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const int n_sm = current_sm_count();
   const int items = (p.n_bins + kHsBins - 1) / kHsBins * 2;
-  kern<<<items < n_sm ? items : n_sm, 32 * (NW + 1), smem, s>>>(p, m);
-  return cudaGetLastError();
+  return launch_kernel(kern, dim3(items < n_sm ? items : n_sm), dim3(32 * (NW + 1)), smem, s, pdl, p, m);
 }
 
-cudaError_t launch_hsum(const HsumParams &p, const HsumMaps &m, cudaStream_t s) {
+cudaError_t launch_hsum(const HsumParams &p, const HsumMaps &m, cudaStream_t s, bool pdl) {
   const bool few = p.n_planes <= 8;
   switch (hsum_warps(p.half)) {
     case 6:
-      if (p.lean) return launch_hsum_t<8, 6, 3, 2>(p, m, s);
-      return few ? launch_hsum_t<8, 6, 5, 1>(p, m, s) : launch_hsum_t<16, 6, 5, 1>(p, m, s);
+      if (p.lean) return launch_hsum_t<8, 6, 3, 2>(p, m, s, pdl);
+      return few ? launch_hsum_t<8, 6, 5, 1>(p, m, s, pdl) : launch_hsum_t<16, 6, 5, 1>(p, m, s, pdl);
     case 11:
       // lean: 2 stages and a register budget that fits next to one FT-convolution CTA
-      if (p.lean) return launch_hsum_t<8, 11, 2, 2>(p, m, s);
-      return few ? launch_hsum_t<8, 11, 3, 1>(p, m, s) : launch_hsum_t<16, 11, 3, 1>(p, m, s);
-    default: return launch_hsum_t<16, 16, 2, 1>(p, m, s);
+      if (p.lean) return launch_hsum_t<8, 11, 2, 2>(p, m, s, pdl);
+      return few ? launch_hsum_t<8, 11, 3, 1>(p, m, s, pdl) : launch_hsum_t<16, 11, 3, 1>(p, m, s, pdl);
+    default: return launch_hsum_t<16, 16, 2, 1>(p, m, s, pdl);
   }
 }
 
@@ -1151,23 +1159,21 @@ cudaError_t launch_split_taps(double2 *taps, long long n, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_recheck(const RecheckParams &p, cudaStream_t s) {
-  recheck_kernel<<<4 * current_sm_count(), 32 * 8, 0, s>>>(p);
-  return cudaGetLastError();
+cudaError_t launch_recheck(const RecheckParams &p, cudaStream_t s, bool pdl) {
+  return launch_kernel(recheck_kernel, dim3(4 * current_sm_count()), dim3(32 * 8), 0, s, pdl, p);
 }
 
-cudaError_t launch_select(const SelectParams &p, cudaStream_t s) {
+cudaError_t launch_select(const SelectParams &p, cudaStream_t s, bool pdl) {
   const int n_sm = current_sm_count();
   const int hsmem = p.n_planes * kSelBuckets * 4;
   cudaError_t e = cudaFuncSetAttribute(select_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hsmem);
   if (e != cudaSuccess) return e;
-  select_hist_kernel<<<n_sm, 1024, hsmem, s>>>(p);
-  select_gather_kernel<<<4 * n_sm, 256, 0, s>>>(p);
+  if ((e = launch_kernel(select_hist_kernel, dim3(n_sm), dim3(1024), hsmem, s, pdl, p)) != cudaSuccess) return e;
+  if ((e = launch_kernel(select_gather_kernel, dim3(4 * n_sm), dim3(256), 0, s, pdl, p)) != cudaSuccess) return e;
   const int fsmem = (kSortCap + kMaxCompat) * (8 + 4);
   e = cudaFuncSetAttribute(select_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fsmem);
   if (e != cudaSuccess) return e;
-  select_finalize_kernel<<<dim3(p.n_planes, kFinSlices), 1024, fsmem, s>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(select_finalize_kernel, dim3(p.n_planes, kFinSlices), dim3(1024), fsmem, s, pdl, p);
 }
 
 }  // namespace fdas
