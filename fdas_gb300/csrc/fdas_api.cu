@@ -102,7 +102,8 @@ struct fdas_handle {
   void *log_user = nullptr;
   float2 *d_twiddle = nullptr;
   double2 *d_twiddle64 = nullptr;
-  float2 *d_series_tw = nullptr;  // e^(-i pi x / N), made on first use
+  float4 *d_series_tw = nullptr;  // twiddle tables of the series FFT, made on first use
+  int series_tw_n = 0;            // for this N
   // fdas_reshape: first template row in use, and the sizes the buffers were allocated for
   int row0 = 0;
   int rc_cap = kRecheckCap;  // entries of the near-threshold recheck list
@@ -936,20 +937,28 @@ fdas_status fdas_series_to_spectrum(fdas_handle *h, const float *samples, uint64
   // ft_conv.py:125-132: at least 2 N samples; extra samples are ignored
   if (n_samples < 2 * (uint64_t)h->N)
     return fail(h, FDAS_ERR_INVALID_ARG, "the series needs at least 2 x n_frequency_bins samples");
-  int radix[64];
-  if (series_radices(h->N, radix, 64) < 0)
+  SeriesPass pass[16];
+  if (series_plan(h->N, pass, 16) < 0)
     return fail(h, FDAS_ERR_UNSUPPORTED, "n_frequency_bins must factor into 2, 3, 5 and 7 for the series FFT");
   BufferSet &S = h->set[ab];
   if (S.pending)
     return fail(h, FDAS_ERR_STATE, "buffer set holds a pending harmonic summing (sync_pipeline); end the pipeline first");
   CK(h, cudaSetDevice(h->cfg.device));
-  if (!h->d_series_tw) {
-    CK(h, cudaMalloc(&h->d_series_tw, sizeof(float2) * (size_t)h->N));
+  if (h->series_tw_n != h->N) {
+    if (!h->d_series_tw)  // (a reshape only makes N smaller)
+      CK(h, cudaMalloc(&h->d_series_tw, sizeof(float4) * series_twiddle_count(h->alloc_N)));
+    h->series_tw_n = 0;
+    CK(h, cudaDeviceSynchronize());  // the other set may still read the table
     CK(h, launch_series_twiddles(h->d_series_tw, h->N, S.stream));
+    h->series_tw_n = h->N;
   }
-  CK(h, cudaMemcpyAsync(S.d_input, samples, sizeof(float) * 2 * (size_t)h->N,
-                        samples_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, S.stream));
+  // device samples are read where they are (as pairs, so 8-byte aligned ones)
+  const bool in_place = samples_on_device && reinterpret_cast<uintptr_t>(samples) % sizeof(float2) == 0;
+  if (!in_place)
+    CK(h, cudaMemcpyAsync(S.d_input, samples, sizeof(float) * 2 * (size_t)h->N,
+                          samples_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, S.stream));
   SeriesParams p{};
+  p.samples = in_place ? reinterpret_cast<const float2 *>(samples) : S.d_input;
   p.z = S.d_input;
   p.scratch = S.d_tiles;  // n_tiles x 2048 >= N complex
   p.tw = h->d_series_tw;

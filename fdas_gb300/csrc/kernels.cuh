@@ -236,15 +236,27 @@ struct TapsParams {
 
 // ---- upstream: spectrum of a real series (ft_conv.py:134-143)
 struct SeriesParams {
-  float2 *z;              // N complex: the 2N samples on entry, the N-bin spectrum on exit
+  const float2 *samples;  // the 2N samples as N complex values (p.z, or the caller's device memory: only read)
+  float2 *z;              // N complex: the N-bin spectrum on exit
   float2 *scratch;        // N complex
-  const float2 *tw;       // e^(-i pi x / N), x < N
+  const float4 *tw;       // series_twiddle_count(n) entries
   int n;                  // N
   float scale;            // applied to every output bin (1 / (2N) in ft_conv.py)
 };
-// radix sequence of an N-point mixed-radix FFT (8, 4, 2, 3, 5, 7); -1 if N has another factor
-int series_radices(int n, int *radix, int max_passes);
-cudaError_t launch_series_twiddles(float2 *tw, int n, cudaStream_t s);
+// one pass of an N-point FFT: radix R over columns j < m = N / R, ns = product of
+// the radices before; in steps of radix[] inside a CTA of B columns
+struct SeriesPass {
+  int R, m, ns;
+  int unit;               // 2N / (ns R): table steps per twiddle exponent
+  int B, log_b;
+  int n_steps;
+  int radix[8];
+};
+constexpr int kTwFine = 2048;  // entries of the fine twiddle table
+// passes of an N-point FFT; -1 if N has a factor other than 2, 3, 5, 7
+int series_plan(int n, SeriesPass *pass, int max_passes);
+size_t series_twiddle_count(int n);
+cudaError_t launch_series_twiddles(float4 *tw, int n, cudaStream_t s);
 cudaError_t launch_series_spectrum(const SeriesParams &p, cudaStream_t s);
 
 cudaError_t launch_tile_fft(const TileParams &p, cudaStream_t s, bool pdl = false);

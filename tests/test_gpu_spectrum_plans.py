@@ -1,0 +1,52 @@
+"""Series FFT over the plans its lengths get (one to several passes of composite
+radix, ragged last columns, every small radix), from host memory, device memory
+and device memory that is not aligned to a pair of samples, and after a reshape;
+against FP64 with the tolerance of the spectrum tests."""
+import io
+
+import numpy as np
+import pytest
+
+from gpu_util import make_pipeline
+from fdas_gb300.fdas import FDAS
+from test_gpu_spectrum import SPEC_TOL
+
+pytestmark = pytest.mark.gpu
+
+
+def check(x, s, n):
+    exact = np.fft.fft(s[:2 * n].astype(np.float64))[:n]
+    rms = np.sqrt(np.mean(np.abs(exact) ** 2))
+    assert np.abs(x - exact).max() <= SPEC_TOL * rms * max(1.0, np.log2(max(n, 2)) / 11)
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 6, 16, 49, 512, 525, 1024, 2187, 16807, 32768, 59049,
+                               65536, 117649, 390625, 786432, 1000000])
+def test_plans(n):
+    import torch
+    s = np.random.default_rng(n).standard_normal(2 * n + 1).astype(np.float32)
+    p = make_pipeline(n, log=io.StringIO(), n_templates=3)
+    out = np.zeros(n, dtype=np.complex64)
+    assert p.series_to_spectrum(s, FDAS.A, scale=1.0, spectrum=out), p.last_error
+    check(out, s, n)
+    d = torch.from_numpy(s).cuda()
+    dev = np.zeros(n, dtype=np.complex64)
+    assert p.series_to_spectrum(d, FDAS.B, scale=1.0, spectrum=dev), p.last_error
+    assert np.array_equal(out, dev)
+    assert torch.equal(d.cpu(), torch.from_numpy(s))  # the caller's samples are only read
+    odd = torch.empty(2 * n + 2, dtype=torch.float32, device="cuda")[1:]
+    odd.copy_(d)
+    assert odd.data_ptr() % 8 == 4
+    assert p.series_to_spectrum(odd, FDAS.A, scale=1.0, spectrum=dev), p.last_error
+    assert np.array_equal(out, dev)
+
+
+def test_after_reshape():
+    n = 9000
+    s = np.random.default_rng(3).standard_normal(2 * n).astype(np.float32)
+    p = make_pipeline(n, log=io.StringIO(), n_templates=3)
+    for m in (9000, 4096, 9000):
+        assert p.reshape(m), p.last_error
+        out = np.zeros(m, dtype=np.complex64)
+        assert p.series_to_spectrum(s, FDAS.A, scale=1.0, spectrum=out), p.last_error
+        check(out, s, m)
