@@ -39,7 +39,9 @@ constexpr int kCtrlBound = kCtrlItems + 1;           // + plane: boundary record
 constexpr int kCtrlWords = kCtrlBound + kMaxPlanes;   // zeroed before every harmonic summing
 constexpr int kCtrlFtcStatus = kCtrlWords;           // FT-convolution status, zeroed before each FT convolution
 constexpr int kCtrlTileStatus = kCtrlWords + 1;      // tiling status (tensor-core form), zeroed before each tiling
-constexpr int kCtrlStride = kCtrlWords + 2;          // control words per buffer set
+constexpr int kCtrlZeroed = kCtrlWords + 2;           // words a search starts from zero
+constexpr int kCtrlStamp = (kCtrlZeroed + 1) & ~1;   // three 64-bit times: start of tiling, FT convolution, harmonic summing
+constexpr int kCtrlStride = kCtrlStamp + 6;          // control words per buffer set
 constexpr uint32_t kDefaultCapacity = 1u << 22;     // candidate records per buffer set
 constexpr uint32_t kMaxCapacity = 1u << 27;
 constexpr int kRecheckCap = 65536;
@@ -88,6 +90,8 @@ struct BufferSet {
   cudaEvent_t ev_hsum = nullptr;  // end of this set's last harmonic-summing kernel
   bool ev_hsum_recorded = false;
   bool input_from_host = false;   // the current spectrum was copied in from host memory
+  bool stamped = false;           // the last search was enqueued in one go: ev[2], ev[3] are times in the control words
+  bool used = false;              // a search or stage ran on this set
 };
 
 }  // namespace
@@ -271,6 +275,7 @@ fdas_status enqueue_input(fdas_handle *h, int ab, const fdas_complex *input, boo
   // NULL: the spectrum that fdas_series_to_spectrum left in this set
   if (!input && !(S.series_spectrum && !device_ptr))
     return fail(h, FDAS_ERR_INVALID_ARG, "input is NULL and no spectrum was made on this buffer set");
+  S.used = true;
   CK(h, cudaEventRecord(S.ev[0], S.stream));
   if (h->cfg.sync_pipeline && h->set[1 - ab].ev_ftc_recorded)
     CK(h, cudaStreamWaitEvent(S.stream, h->set[1 - ab].ev[3], 0));  // FDAS.cpp:287-288
@@ -288,6 +293,10 @@ fdas_status enqueue_input(fdas_handle *h, int ab, const fdas_complex *input, boo
   CK(h, cudaEventRecord(S.ev[1], S.stream));
   S.have_input = true;
   return FDAS_OK;
+}
+
+unsigned long long *stamp_at(const BufferSet &S, int i) {
+  return reinterpret_cast<unsigned long long *>(S.d_ctrl + kCtrlStamp) + i;
 }
 
 // `chain`: the stages of one search are enqueued in one go (not a stage call, not
@@ -323,11 +332,15 @@ fdas_status enqueue_tiling(fdas_handle *h, int ab, bool chain) {
   } else {
     if (chain) {
       p.zero = S.d_ctrl;
-      p.n_zero = kCtrlStride;
+      p.n_zero = kCtrlZeroed;
+      p.stamp = stamp_at(S, 0);
     }
     CK(h, launch_tile_fft(p, S.stream));
   }
-  CK(h, cudaEventRecord(S.ev[2], S.stream));
+  // an event between two kernels keeps the second from starting early (about 2 us
+  // each): in a chain the kernels write down their start times instead
+  S.stamped = chain;
+  if (!chain) CK(h, cudaEventRecord(S.ev[2], S.stream));
   return FDAS_OK;
 }
 
@@ -366,15 +379,17 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which, bool chain)
   if (S.input_from_host && !h->cfg.overlap && !h->cfg.sync_pipeline && h->set[1 - ab].ev_hsum_recorded)
     CK(h, cudaStreamWaitEvent(S.stream, h->set[1 - ab].ev_hsum, 0));
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl + kCtrlFtcStatus, 0, sizeof(unsigned), S.stream));
+  if (chain) p.stamp = stamp_at(S, 1);
   CK(h, launch_ftc(p, S.stream, chain));
-  CK(h, cudaEventRecord(S.ev[3], S.stream));
+  if (!chain) CK(h, cudaEventRecord(S.ev[3], S.stream));
   S.ftc_unchecked = true;
   S.ev_ftc_recorded = true;
   S.fop_from_input = true;
   return FDAS_OK;
 }
 
-fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_part which, bool chain) {
+fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_part which, bool chain,
+                         uint32_t *loc = nullptr, float *pwr = nullptr) {
   BufferSet &S = h->set[ab];
   const float *thr = thr_in;
   if (!thr) {
@@ -426,8 +441,10 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   if (hsum_smem_bytes(p) > 227 * 1024)
     return fail(h, FDAS_ERR_UNSUPPORTED, "harmonic summing staging exceeds shared memory (too many templates x planes)");
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl, 0, sizeof(unsigned) * kCtrlWords, S.stream));
+  if (chain) p.stamp = stamp_at(S, 2);
   CK(h, launch_hsum(p, S.maps, S.stream, chain));
-  if (S.ev_hsum) {  // (the batched form's per-trial views have none)
+  // (the batched form's per-trial views have none; with one set in use nobody waits for it)
+  if (S.ev_hsum && (!chain || h->set[1 - ab].used)) {
     CK(h, cudaEventRecord(S.ev_hsum, S.stream));
     S.ev_hsum_recorded = true;
   }
@@ -470,18 +487,37 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   f.compat_pwr = S.d_cpwr;
   f.invalid_location = (uint32_t)((h->H + 1 + h->H) & 0x7f) << 22;  // encode(1, H+1, 0), gen_info.h:69
   f.status = p.status;
+  f.ctrl = S.d_ctrl;
+  f.host_ctrl = S.h_ctrl;
+  f.n_ctrl = kCtrlStride;
+  f.host_loc = loc;
+  f.host_pwr = pwr;
   CK(h, launch_select(f, S.stream, chain));
-  CK(h, cudaMemcpyAsync(S.h_ctrl, S.d_ctrl, sizeof(unsigned) * kCtrlStride, cudaMemcpyDeviceToHost, S.stream));
   CK(h, cudaEventRecord(S.ev[4], S.stream));
   S.ctrl_valid = true;
   return FDAS_OK;
 }
 
-fdas_status enqueue_download(fdas_handle *h, int ab, uint32_t *loc, float *pwr) {
+// The candidate list of a search goes into the caller's arrays by the selection's
+// last kernel where they are pinned (two copies less at the end of a search), else
+// by copies.
+bool pinned(const void *ptr) {
+  cudaPointerAttributes at{};
+  if (!ptr || cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeHost && at.devicePointer == ptr;
+}
+fdas_status enqueue_hsum_download(fdas_handle *h, int ab, const float *thr, fdas_fop_part which, bool chain, uint32_t *loc,
+                                  float *pwr) {
   BufferSet &S = h->set[ab];
   const size_t n = (size_t)h->P * h->per_plane;
-  if (loc) CK(h, cudaMemcpyAsync(loc, S.d_cloc, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, S.stream));
-  if (pwr) CK(h, cudaMemcpyAsync(pwr, S.d_cpwr, sizeof(float) * n, cudaMemcpyDeviceToHost, S.stream));
+  const bool direct = pinned(loc) && pinned(loc + n - 1) && pinned(pwr) && pinned(pwr + n - 1);
+  fdas_status st = enqueue_hsum(h, ab, thr, which, chain, direct ? loc : nullptr, direct ? pwr : nullptr);
+  if (st != FDAS_OK) return st;
+  if (loc && !direct) CK(h, cudaMemcpyAsync(loc, S.d_cloc, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, S.stream));
+  if (pwr && !direct) CK(h, cudaMemcpyAsync(pwr, S.d_cpwr, sizeof(float) * n, cudaMemcpyDeviceToHost, S.stream));
   CK(h, cudaEventRecord(S.ev[5], S.stream));
   S.launched = true;
   return FDAS_OK;
@@ -491,9 +527,7 @@ fdas_status release_pending(fdas_handle *h, int ab) {
   BufferSet &S = h->set[ab];
   if (!S.pending) return FDAS_OK;
   S.pending = false;
-  fdas_status st = enqueue_hsum(h, ab, S.p_thr.data(), S.p_which, false);
-  if (st != FDAS_OK) return st;
-  return enqueue_download(h, ab, S.p_loc, S.p_pwr);
+  return enqueue_hsum_download(h, ab, S.p_thr.data(), S.p_which, false, S.p_loc, S.p_pwr);
 }
 
 // Device-side timeouts of the last search on set `ab`, once its stream has
@@ -530,6 +564,19 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
     return -1.f;
   }
   return ms;
+}
+
+// ms of tiling, FT convolution and harmonic summing of a completed search
+void stage_times(const BufferSet &S, float *ms3) {
+  if (!S.stamped) {
+    for (int i = 0; i < 3; ++i) ms3[i] = elapsed(S.ev[1 + i], S.ev[2 + i]);
+    return;
+  }
+  unsigned long long t[3];
+  std::memcpy(t, S.h_ctrl + kCtrlStamp, sizeof(t));
+  ms3[0] = (float)(1e-6 * (double)(long long)(t[1] - t[0]));
+  ms3[1] = (float)(1e-6 * (double)(long long)(t[2] - t[1]));
+  ms3[2] = std::max(0.f, elapsed(S.ev[1], S.ev[4]) - ms3[0] - ms3[1]);
 }
 
 void free_set(BufferSet &S) {
@@ -907,6 +954,8 @@ fdas_status fdas_perform_ft_convolution(fdas_handle *h, fdas_fop_part which, fda
   CHECK_SET(h, ab);
   if (!valid_part(which)) return fail(h, FDAS_ERR_INVALID_ARG, "invalid FOP part");
   CK(h, cudaSetDevice(h->cfg.device));
+  if (h->set[ab].stamped) CK(h, cudaEventRecord(h->set[ab].ev[2], h->set[ab].stream));
+  h->set[ab].stamped = false;
   fdas_status st = enqueue_ftc(h, ab, which, false);
   if (st != FDAS_OK) return st;
   if ((st = sync_set(h, ab)) != FDAS_OK) return st;
@@ -921,6 +970,9 @@ fdas_status fdas_perform_harmonic_summing(fdas_handle *h, const float *threshold
   if (!valid_part(which)) return fail(h, FDAS_ERR_INVALID_ARG, "invalid FOP part");
   CK(h, cudaSetDevice(h->cfg.device));
   BufferSet &S = h->set[ab];
+  S.used = true;
+  if (S.stamped) CK(h, cudaEventRecord(S.ev[2], S.stream));
+  S.stamped = false;
   CK(h, cudaEventRecord(S.ev[3], S.stream));
   fdas_status st = enqueue_hsum(h, ab, thresholds, which, false);
   if (st != FDAS_OK) return st;
@@ -1006,10 +1058,9 @@ fdas_status fdas_launch(fdas_handle *h, const fdas_complex *input, const float *
     S.launched = true;
     t[3] = t[4] = steady_ns();  // harmonic summing and download are enqueued later
   } else {
-    if ((st = enqueue_hsum(h, ab, thresholds, which, chain)) != FDAS_OK) return st;
-    t[3] = steady_ns();
-    if ((st = enqueue_download(h, ab, detection_location, detection_power)) != FDAS_OK) return st;
-    t[4] = steady_ns();
+    if ((st = enqueue_hsum_download(h, ab, thresholds, which, chain, detection_location, detection_power)) != FDAS_OK)
+      return st;
+    t[3] = t[4] = steady_ns();  // (one step: the list is written by harmonic summing's last kernel)
   }
   if (h->cfg.trace_enqueue) {
     // FDAS.cpp:567-575: whole milliseconds of the enqueue steps, then the raw times
@@ -1033,8 +1084,7 @@ fdas_status fdas_enqueue_search_device(fdas_handle *h, const fdas_complex *d_inp
   if ((st = enqueue_input(h, ab, d_input, true)) != FDAS_OK) return st;
   if ((st = enqueue_tiling(h, ab, chain)) != FDAS_OK) return st;
   if ((st = enqueue_ftc(h, ab, which, chain)) != FDAS_OK) return st;
-  if ((st = enqueue_hsum(h, ab, thresholds, which, chain)) != FDAS_OK) return st;
-  return enqueue_download(h, ab, nullptr, nullptr);
+  return enqueue_hsum_download(h, ab, thresholds, which, chain, nullptr, nullptr);
 }
 
 fdas_status fdas_synchronize(fdas_handle *h, fdas_buffer_set ab) {
@@ -1241,10 +1291,12 @@ fdas_status fdas_get_stage_times(fdas_handle *h, fdas_buffer_set ab, float *ms6)
   BufferSet &S = h->set[ab];
   CK(h, cudaSetDevice(h->cfg.device));
   CK(h, cudaEventSynchronize(S.ev[5]));
+  float st[3];
+  stage_times(S, st);
   ms6[0] = elapsed(S.ev[0], S.ev[1]);
-  ms6[1] = elapsed(S.ev[1], S.ev[2]);
-  ms6[2] = elapsed(S.ev[2], S.ev[3]);
-  ms6[3] = elapsed(S.ev[3], S.ev[4]);
+  ms6[1] = st[0];
+  ms6[2] = st[1];
+  ms6[3] = st[2];
   ms6[4] = elapsed(S.ev[4], S.ev[5]);
   ms6[5] = elapsed(S.ev[0], S.ev[5]);
   return FDAS_OK;
@@ -1290,9 +1342,11 @@ void fdas_print_stats(fdas_handle *h, fdas_buffer_set ab, int reset) {
   const char set_c = ab == FDAS_SET_A ? 'A' : 'B';
   logf(h, "[INFO] Launch  #%u%c complete @ %.3f ms II ~ %.3f ms", h->pipeline_launches, set_c, acc * 1e-6,
        (acc - h->pipeline_accum_ns) * 1e-6);
-  logf(h, "[INFO]   Preparation duration: %.3f ms", elapsed(S.ev[1], S.ev[2]));
-  logf(h, "[INFO]   FT convolution and IFFT duration: %.3f ms", elapsed(S.ev[2], S.ev[3]));
-  logf(h, "[INFO]   Harmonic summing duration: %.3f ms", elapsed(S.ev[3], S.ev[4]));
+  float st[3];
+  stage_times(S, st);
+  logf(h, "[INFO]   Preparation duration: %.3f ms", st[0]);
+  logf(h, "[INFO]   FT convolution and IFFT duration: %.3f ms", st[1]);
+  logf(h, "[INFO]   Harmonic summing duration: %.3f ms", st[2]);
   logf(h, "[INFO]   Total duration: %.3f ms", elapsed(S.ev[0], S.ev[5]));
   h->pipeline_accum_ns = acc;
 }
@@ -1308,7 +1362,14 @@ void fdas_print_events(fdas_handle *h, fdas_buffer_set ab) {
   // convolution, harmonic summing and candidate transfer; each stage starts
   // where the one before it ends on the set's stream
   long long t[6];
-  for (int i = 0; i < 6; ++i) t[i] = event_ns(h, S.ev[i]);
+  for (int i = 0; i < 6; ++i)
+    if (!S.stamped || (i != 2 && i != 3)) t[i] = event_ns(h, S.ev[i]);
+  if (S.stamped) {
+    float st[3];
+    stage_times(S, st);
+    t[2] = std::min(t[4], t[1] + (long long)llround(1e6 * (double)st[0]));
+    t[3] = std::min(t[4], t[2] + (long long)llround(1e6 * (double)st[1]));
+  }
   logf(h, "@@@,%c,%lld,%lld,%lld,%lld,%lld,%lld,%lld,%lld,%lld,%lld", ab == FDAS_SET_A ? 'A' : 'B', t[0], t[1], t[1],
        t[2], t[2], t[3], t[3], t[4], t[4], t[5]);
 }

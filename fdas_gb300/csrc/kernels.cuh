@@ -41,10 +41,15 @@ __host__ __device__ inline unsigned long long cand_key(int plane, int row, int b
 // grid_release() (or by ending).  Both do nothing without the launch attribute.
 // Hides launch latency and prologues, which bound short spectra: the
 // allocation-free FT convolution of 4096 bins 18.5 -> 14.2 us, of 100003 x 43 rows
-// 28.8 -> 22.7, a search of 32768 bins 94.8 -> 83.7 (events between its stages
-// still hold some kernels back), of 2^21 699 -> 691.
+// 28.8 -> 22.7, a search of 32768 bins 94.8 -> 83.7 us, and to 68.3 without events
+// between its kernels and copies after them, of 2^21 bins 699 -> 691 -> 678.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// %globaltimer (32 ns steps here) written by one thread of a kernel where its
+// part of the search starts, or nothing
+__device__ __forceinline__ void stamp(unsigned long long *at) {
+  if (at && blockIdx.x == 0 && threadIdx.x == 0) asm volatile("mov.u64 %0, %globaltimer;" : "=l"(*at));
+}
 template <typename Kernel, typename... Args>
 cudaError_t launch_kernel(Kernel kern, dim3 grid, dim3 block, int smem, cudaStream_t s, bool pdl, Args... args) {
   cudaLaunchAttribute at{};
@@ -96,6 +101,7 @@ struct TileParams {
   int n_trials = 0;
   unsigned *zero = nullptr;  // words to zero before the following kernels run (a search's control words)
   int n_zero = 0;
+  unsigned long long *stamp = nullptr;  // start time (stage times of a search enqueued in one go)
 };
 
 // ---- (c) template multiply + inverse FFT + |.|^2 + discard (mux_and_mult,
@@ -129,6 +135,7 @@ struct FtcParams {
   // to `tiles_out` as complex spectra
   const float2 *input = nullptr;
   float2 *tiles_out = nullptr;
+  unsigned long long *stamp = nullptr;
 };
 
 // ---- (d) harmonic summing + thresholds + candidate compaction (preload,
@@ -164,6 +171,7 @@ struct HsumParams {
   int lean;               // 1: fewer stages and registers (shares an SM with the FT convolution)
   int inject_stall = 0;   // test hook: the first stage of every CTA is announced on its barriers
                           // but its copies are not issued, so the consumers' waits run out
+  unsigned long long *stamp = nullptr;
 };
 
 // 2-D tensor maps of the FOP (rows x stride floats), one box shape per plane
@@ -210,8 +218,13 @@ struct SelectParams {
   float *sel_pwr;
   uint32_t *compat_loc;   // [plane][per_plane]
   float *compat_pwr;
+  uint32_t *host_loc = nullptr;  // the list once more, in pinned host memory
+  float *host_pwr = nullptr;
   uint32_t invalid_location;
   int *status;
+  const unsigned *ctrl;   // n_ctrl control words, copied to pinned host memory at the end
+  unsigned *host_ctrl;
+  int n_ctrl;
 };
 
 // ---- template spectra / taps in FP64

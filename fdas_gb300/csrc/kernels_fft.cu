@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 3) tile_fft_kernel(TileParams
   grid_release();
   if (blockIdx.x == 0 && p.n_zero) {
     grid_wait();
+    stamp(p.stamp);
     for (int i = threadIdx.x; i < p.n_zero; i += blockDim.x) p.zero[i] = 0u;
   }
   if (tile >= p.n_tiles) return;
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(256, 1) ftc_kernel(FtcParams p) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
+  stamp(p.stamp);
   const TwiddleBases tb = load_twiddle_bases<+1>(p.twiddle, lane);
   if (item < n_items && lane == 0)
     prefetch_template(ex, p.tmpl + (long long)(p.row_begin + item % p.n_rows) * kTile, bar);
@@ -262,6 +264,7 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   fill_twiddle2(twt, p.twiddle);
+  stamp(p.stamp);
   __syncthreads();
   if (item < n_items && tp == 0) {
     if (p.inject_stall) mbar_arrive_expect_tx(bar, kTile * 8);  // test hook: a copy that never comes
@@ -478,6 +481,7 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     grid_wait();
+    stamp(p.stamp);
     if (threadIdx.x == 0)
       for (int i = 0; i < kGroupRing && i < steps; ++i) {
         if (i == 0 && p.inject_stall) {  // test hook: a copy that never comes

@@ -640,6 +640,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
   }
   grid_release();
   grid_wait();
+  stamp(p.stamp);
   __syncthreads();
 
   if (warp == NW) {
@@ -1082,8 +1083,17 @@ __global__ void __launch_bounds__(1024) select_finalize_kernel(SelectParams p) {
   }
   __syncthreads();
   const int kept = keep_a + c;
-  uint32_t *cl = p.compat_loc + (size_t)plane * K;
-  float *cp = p.compat_pwr + (size_t)plane * K;
+  uint32_t *cl = p.compat_loc + (size_t)plane * K, *hl = p.host_loc ? p.host_loc + (size_t)plane * K : nullptr;
+  float *cp = p.compat_pwr + (size_t)plane * K, *hp = p.host_pwr ? p.host_pwr + (size_t)plane * K : nullptr;
+  auto put = [&](int at, uint32_t loc, float pwr) {
+    cl[at] = loc;
+    cp[at] = pwr;
+    if (hl) hl[at] = loc;
+    if (hp) hp[at] = pwr;
+  };
+  // the control words are final: the kernels before have ended
+  if (blockIdx.x == 0 && blockIdx.y == 0)
+    for (int i = threadIdx.x; i < p.n_ctrl; i += blockDim.x) p.host_ctrl[i] = p.ctrl[i];
   // this CTA's slice [lo, hi) of the K entries: the kept records i in it are
   // placed, the unused positions in it (i >= kept) padded
   const int per = (K + (int)gridDim.y - 1) / (int)gridDim.y;
@@ -1099,13 +1109,11 @@ __global__ void __launch_bounds__(1024) select_finalize_kernel(SelectParams p) {
     if (lane == 0) {
       const unsigned row = (unsigned)(ki >> 32) & 0xffffu, bin = (unsigned)(ki & 0xffffffffu);
       // gen_info.h:62-64: ((h-1)&7)<<29 | (row&0x7f)<<22 | (bin&0x3fffff)
-      cl[pos] = (((unsigned)plane & 7u) << 29) | ((row & 0x7fu) << 22) | (bin & 0x3fffffu);
-      cp[pos] = finp[i];
+      put((int)pos, (((unsigned)plane & 7u) << 29) | ((row & 0x7fu) << 22) | (bin & 0x3fffffu), finp[i]);
     }
   }
   for (int i = max(lo, kept) + (int)threadIdx.x; i < hi; i += blockDim.x) {
-    cl[i] = p.invalid_location;
-    cp[i] = -1.0f;
+    put(i, p.invalid_location, -1.0f);
   }
 }
 

@@ -91,3 +91,22 @@ def test_noalloc_in_a_graph():
     assert call(plain) == _lib.OK
     torch.cuda.synchronize()
     assert torch.equal(plain, graphed)
+
+
+@pytest.mark.parametrize("pins", [(True, True), (True, False), (False, True), (False, False)])
+def test_list_into_pinned_and_pageable_arrays(pins):
+    """The selection writes pinned arrays itself, others are copied to: the same list."""
+    from fdas_gb300.fdas import PinnedArray
+    n, thr = 20000, O.chi2_thresholds(1e-4, 8)
+    p = handle(n)
+    nc = p.get_candidate_list_sz()
+    keep = [PinnedArray((nc,), d) if pin else None for pin, d in zip(pins, (np.uint32, np.float32))]
+    loc, pwr = (k.array if k else np.empty(nc, d) for k, d in zip(keep, (np.uint32, np.float32)))
+    loc[:], pwr[:] = 7, 7
+    for seed in (1, 2):
+        assert p.launch(spectrum(n, seed), thr, loc, pwr, FDAS.AllAccelerations, FDAS.A) and p.wait(FDAS.A)
+        want_loc, want_pwr = np.zeros(nc, np.uint32), np.zeros(nc, np.float32)
+        assert p.retrieve_candidates(want_loc, want_pwr, FDAS.A)
+        assert np.array_equal(loc, want_loc) and np.array_equal(pwr, want_pwr)
+        ms = p.stage_times(FDAS.A)
+        assert (ms >= 0).all() and ms[1] > 0 and ms[2] > 0 and ms[3] > 0 and ms[:5].sum() <= ms[5] + 0.05
