@@ -12,11 +12,7 @@
 //   so lane l ends with outputs n = l + 32 c + 64 d (c in {0,1}, d in [0,32)):
 //   for fixed (c, d) the 32 lanes hold 32 consecutive outputs.
 //
-//   forward (sign -1) is the mirror image: natural-order input x[m + 64 d] is
-//   loaded with lane l holding m in {l, l+32}; DFT32 over d, twiddle
-//   w^(-m kappa), exchange, DFT64 over m; lane kappa ends with X[32 k' + kappa].
-//
-// Global loads and stores of both directions are therefore unit-stride across
+// Global loads and stores are therefore unit-stride across
 // the warp, which makes every access coalesced without any permutation of the
 // spectra in memory.  The FPGA reference uses a radix-2^2 streaming engine with
 // bit-reversed output instead (fft_4p.cl); only the transform is shared.
@@ -240,12 +236,15 @@ __device__ __forceinline__ void dft_composite(float2 *v) {
   });
 }
 
-// Register slot of output k for the 64 = 8x8 and 32 = 4x8 transforms.
+// Register slot of output k for the 64 = 8x8, 32 = 4x8 and 16 = 4x4 transforms.
+__host__ __device__ constexpr int pos16(int k) { return 4 * (k % 4) + k / 4; }
 __host__ __device__ constexpr int pos64(int k) { return 8 * (k % 8) + k / 8; }
 __host__ __device__ constexpr int pos32(int k) { return 8 * (k % 4) + k / 4; }
 
 template <int S, int OFF>
 __device__ __forceinline__ void dft64(float2 *v) { dft_composite<S, 8, 8, OFF, 1>(v); }
+template <int S, int OFF>
+__device__ __forceinline__ void dft16(float2 *v) { dft_composite<S, 4, 4, OFF, 1>(v); }
 template <int S, int OFF>
 __device__ __forceinline__ void dft32(float2 *v) { dft_composite<S, 4, 8, OFF, 1>(v); }
 
@@ -326,49 +325,6 @@ __device__ __forceinline__ void ifft2048_core(float2 *v, const TwiddleBases &tb,
   after_exchange();
   dft32<+1, 0>(v);
   dft32<+1, 32>(v);
-}
-
-// Forward transform core: v[32 c + d] holds x[lane + 32 c + 64 d] on entry.
-// On exit v[pos64(k')] holds X[32 k' + lane].
-__device__ __forceinline__ void fft2048_core(float2 *v, const TwiddleBases &tb, float *ex, int lane) {
-  dft32<-1, 0>(v);
-  dft32<-1, 32>(v);
-  // twiddle: U_m[kappa] * w^(-m kappa), m = lane + 32 c, kappa = klo + 8 khi.
-  // w^(-(lane + 32c) kappa) = w^(-lane kappa) * e^(-2 pi i c kappa / 64)
-  // per-lane part from the bases: kappa = klo + 8 khi -> lo[klo] * hi[khi]
-  sfor<2>([&](auto C) {
-    constexpr int c = decltype(C)::value;
-    sfor<32>([&](auto K) {
-      constexpr int kap = decltype(K)::value;
-      constexpr int klo = kap % 8, khi = kap / 8;
-      constexpr int idx = 32 * c + pos32(kap);
-      float2 t = v[idx];
-      if constexpr (klo != 0 && khi != 0) t = cmul(t, cmul(tb.lo[klo], tb.hi[khi]));
-      else if constexpr (klo != 0) t = cmul(t, tb.lo[klo]);
-      else if constexpr (khi != 0) t = cmul(t, tb.hi[khi]);
-      if constexpr (c == 1) t = rot<-1, 64, kap>(t);
-      v[idx] = t;
-    });
-  });
-  // exchange: column writes (8-byte), row reads (16-byte)
-  float2 *col = reinterpret_cast<float2 *>(ex);
-  sfor<2>([&](auto C) {
-    constexpr int c = decltype(C)::value;
-    sfor<32>([&](auto K) {
-      constexpr int kap = decltype(K)::value;
-      col[kExPitch * kap + lane + 32 * c] = v[32 * c + pos32(kap)];
-    });
-  });
-  __syncwarp();
-  const float4 *row = reinterpret_cast<const float4 *>(ex + 2 * kExPitch * lane);
-  sfor<32>([&](auto P) {
-    constexpr int p = decltype(P)::value;
-    float4 q = row[p];
-    v[2 * p] = make_float2(q.x, q.y);
-    v[2 * p + 1] = make_float2(q.z, q.w);
-  });
-  __syncwarp();
-  dft64<-1, 0>(v);
 }
 
 }  // namespace fdas
@@ -542,9 +498,6 @@ __device__ __forceinline__ void bfly(float2 &a, float2 &b, float2 t) {
   b = f2_fma(make_float2(-2.f, -2.f), a, p);
   a = p;
 }
-// the same with i t
-__device__ __forceinline__ void bfly_i(float2 &a, float2 &b, float2 t) { bfly(a, b, make_float2(-t.y, t.x)); }
-
 // the second output from the inputs instead: where the first output is much the
 // larger one (a signal's peak), its rounding does not reach the second
 __device__ __forceinline__ void bfly_direct(float2 &a, float2 &b, float2 t) {
@@ -557,29 +510,28 @@ __device__ __forceinline__ void bfly_direct(float2 &a, float2 &b, float2 t) {
 __host__ __device__ constexpr int rev3(int k) { return ((k & 1) << 2) | (k & 2) | ((k >> 2) & 1); }
 
 // x[i] -> (-1)^popcount(k) sum_i x[i] z^i e^(2 pi i i k / 8) at x[rev3(k)].
-// LAST: the transform's last stage, outputs not taken from one another (2 us of
-// 314 at 2^21 bins x 85 rows; in every stage: 31 us).
+// LAST: the transform's last DFT8, where a signal's peak and its weak neighbours
+// part: the outputs of its last two stages are not taken from one another (8 us of
+// 308 at 2^21 bins x 85 rows; in every stage of both DFT8: 32 us).
 template <bool LAST>
 __device__ __forceinline__ void twisted_dft8(float2 *x, const TwistedTw &t) {
   bfly(x[0], x[4], t.t4);
   bfly(x[1], x[5], t.t4);
   bfly(x[2], x[6], t.t4);
   bfly(x[3], x[7], t.t4);
-  bfly(x[0], x[2], t.t2);
-  bfly(x[1], x[3], t.t2);
-  bfly_i(x[4], x[6], t.t2);
-  bfly_i(x[5], x[7], t.t2);
-  if constexpr (LAST) {
-    bfly_direct(x[0], x[1], t.t1);
-    bfly_direct(x[2], x[3], make_float2(-t.t1.y, t.t1.x));
-    bfly_direct(x[4], x[5], t.t1p);
-    bfly_direct(x[6], x[7], make_float2(-t.t1p.y, t.t1p.x));
-  } else {
-    bfly(x[0], x[1], t.t1);
-    bfly_i(x[2], x[3], t.t1);
-    bfly(x[4], x[5], t.t1p);
-    bfly_i(x[6], x[7], t.t1p);
-  }
+  auto stage = [](float2 &a, float2 &b, float2 w) {
+    if constexpr (LAST) bfly_direct(a, b, w);
+    else bfly(a, b, w);
+  };
+  auto times_i = [](float2 w) { return make_float2(-w.y, w.x); };
+  stage(x[0], x[2], t.t2);
+  stage(x[1], x[3], t.t2);
+  stage(x[4], x[6], times_i(t.t2));
+  stage(x[5], x[7], times_i(t.t2));
+  stage(x[0], x[1], t.t1);
+  stage(x[2], x[3], times_i(t.t1));
+  stage(x[4], x[5], t.t1p);
+  stage(x[6], x[7], times_i(t.t1p));
 }
 
 // Twiddles of pass 2 of thread tp (m = 16 h + (l & 15), g = l >> 4), as powers

@@ -11,28 +11,32 @@ namespace fdas {
 
 constexpr int kWarpsPerCta = 8;
 
-// One warp per tile.  Tile i covers spectrum bins [i P - O, i P + P): bins
-// below 0 (the first tile's overlap) and from N on (the last tile's padding)
-// read as zero -- tile_input.cl.mako:42-94 / ft_conv.py:165-180.
-// Three warps per CTA and three CTAs per SM (at most 224 registers): 9 warps
-// per SM, so the 1289 tiles of a 2^21-bin search run in a single wave
-// (1368 warp slots) instead of 1216 + 73.
-constexpr int kTileWarps = 3;
+// Four warps per tile, 16 values per thread: 2048 = 16 x 16 x 8, DFT16, DFT16 and
+// two DFT8 with two exchanges through one 16.5 KB buffer.  With n = n0 + 128 n1,
+// n0 = m0 + 8 m1, k = k0 + 16 k1 + 256 k2:
+//   thread n0         Y[n0][k0] = DFT16_n1(x[n0 + 128 n1]) w^(-n0 k0)
+//   thread (m0, k0)   U[m0][k1] = DFT16_m1(Y[m0 + 8 m1][k0]) w^(-16 m0 k1)
+//   thread c, c + 128 X[c + 256 k2] = DFT8_m0(U[m0][k1]), c = k0 + 16 k1
+// so loads and stores are unit-stride.  One warp per tile (64 values a lane) was
+// bound by that warp's chain; tiling at 2^21 / 2^19 / 2^15 bins: 10.3 / 4.8 / 2.7 us
+// against 16.2 / 11.3 / 9.5.  At 2^21 the 1289 CTAs of 8 per SM are one wave and a
+// bit; 17 MB are read and 21 written (5.6 us at the copy rate).  Tile i covers spectrum bins [i P - O,
+// i P + P): bins below 0 (the first tile's overlap) and from N on (the last
+// tile's padding) read as zero -- tile_input.cl.mako:42-94 / ft_conv.py:165-180.
+constexpr int kTileThreads = 128;
+constexpr int kTilePitch = 129;  // odd: the column reads of the first exchange meet no bank twice
 template <bool BATCH>
-__global__ void __launch_bounds__(32 * kTileWarps, 3) tile_fft_kernel(TileParams p) {
-  extern __shared__ float4 smem_f4[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x * kTileWarps + warp;
+__global__ void __launch_bounds__(kTileThreads, 8) tile_fft_kernel(TileParams p) {
+  __shared__ float2 ex[16 * kTilePitch];
+  const int t = threadIdx.x;
+  const int tile = blockIdx.x;
   grid_release();
-  if (blockIdx.x == 0 && p.n_zero) {
-    grid_wait();
-    stamp(p.stamp);
-    for (int i = threadIdx.x; i < p.n_zero; i += blockDim.x) p.zero[i] = 0u;
-  }
-  if (tile >= p.n_tiles) return;
-  float *ex = reinterpret_cast<float *>(smem_f4) + warp * kExFloats;
-  const TwiddleBases tb = load_twiddle_bases<-1>(p.twiddle, lane);
-  float2 v[64];
+  const int m0 = t >> 4, k0 = t & 15;
+  float2 w[16];  // twiddles, there before the tile is
+  sfor<15>([&](auto K) {
+    constexpr int k = decltype(K)::value + 1;
+    w[k] = __ldg(p.twiddle + k * t);  // k t < 2048
+  });
   const float2 *input = p.input;
   int n_bins = p.n_bins;
   long long local = tile;
@@ -42,21 +46,60 @@ __global__ void __launch_bounds__(32 * kTileWarps, 3) tile_fft_kernel(TileParams
     n_bins = tr.n_bins;
     local = tile - tr.tile_begin;
   }
-  const long long start = local * p.payload - p.overlap;
   grid_wait();
+  if (blockIdx.x == 0 && p.n_zero) {
+    stamp(p.stamp);
+    for (int i = t; i < p.n_zero; i += kTileThreads) p.zero[i] = 0u;
+  }
+  const long long start = local * p.payload - p.overlap + t;
+  float2 v[16];
+  sfor<16>([&](auto N1) {
+    constexpr int n1 = decltype(N1)::value;
+    const long long b = start + 128 * n1;
+    v[n1] = (b >= 0 && b < n_bins) ? input[b] : make_float2(0.f, 0.f);
+  });
+  // (the table holds w^j = e^(+2 pi i j / 2048); conjugated here)
+  auto conj_mul = [](float2 a, float2 b) {
+    return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.y, b.x, -a.x * b.y));
+  };
+  dft16<-1, 0>(v);
+  sfor<16>([&](auto K) {
+    constexpr int k = decltype(K)::value;
+    float2 y = v[pos16(k)];
+    if constexpr (k > 0) y = conj_mul(y, w[k]);
+    ex[k * kTilePitch + t] = y;
+  });
+  sfor<15>([&](auto K) {
+    constexpr int k = decltype(K)::value + 1;
+    w[k] = __ldg(p.twiddle + 16 * k * m0);  // < 2048
+  });
+  __syncthreads();
+  sfor<16>([&](auto M1) {
+    constexpr int m1 = decltype(M1)::value;
+    v[m1] = ex[k0 * kTilePitch + m0 + 8 * m1];
+  });
+  __syncthreads();
+  dft16<-1, 0>(v);
+  sfor<16>([&](auto K) {
+    constexpr int k = decltype(K)::value;
+    float2 y = v[pos16(k)];
+    if constexpr (k > 0) y = conj_mul(y, w[k]);
+    ex[256 * m0 + k0 + 16 * k] = y;
+  });
+  __syncthreads();
+  float2 *out = p.tiles + (long long)tile * kTile + t;
   sfor<2>([&](auto C) {
     constexpr int c = decltype(C)::value;
-    sfor<32>([&](auto D) {
-      constexpr int d = decltype(D)::value;
-      const long long b = start + lane + 32 * c + 64 * d;
-      v[32 * c + d] = (b >= 0 && b < n_bins) ? __ldg(input + b) : make_float2(0.f, 0.f);
+    float2 u[8];
+    sfor<8>([&](auto M) {
+      constexpr int m = decltype(M)::value;
+      u[m] = ex[256 * m + 128 * c + t];
     });
-  });
-  fft2048_core(v, tb, ex, lane);
-  float2 *out = p.tiles + (long long)tile * kTile;
-  sfor<64>([&](auto K) {
-    constexpr int k = decltype(K)::value;
-    out[32 * k + lane] = v[pos64(k)];
+    dft8<-1, 0, 1>(u);
+    sfor<8>([&](auto K) {
+      constexpr int k = decltype(K)::value;
+      out[128 * c + 256 * k] = u[k];
+    });
   });
 }
 
@@ -351,7 +394,7 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
 // Bound by the shared-memory pipe and the FMA pipe about alike (2^19 bins x 85
 // rows: 64% and 63% busy, ~600 wavefronts and ~550 FMA-pipe clocks per item of
 // ~880 clocks); the pair form below moves ~960 wavefronts and 680 clocks per
-// item.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 314 / 89 / 17.5 us
+// item.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 308 / 82 / 11.3 us
 // against 432 / 118 / 19.4 us of the pair form.  The same with 6 pairs and the
 // tile in registers (168 a thread) took 361 us, 4 pairs of two rows each 488 us;
 // the twiddle products all packed 336 us, all scalar 345 us.
@@ -672,12 +715,8 @@ int current_sm_count() {
 static int ex_smem_bytes() { return kWarpsPerCta * kExFloats * (int)sizeof(float); }
 
 cudaError_t launch_tile_fft(const TileParams &p, cudaStream_t s, bool pdl) {
-  const int smem = kTileWarps * kExFloats * (int)sizeof(float);
   auto kern = p.trials ? tile_fft_kernel<true> : tile_fft_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  dim3 grid((p.n_tiles + kTileWarps - 1) / kTileWarps);
-  return launch_kernel(kern, grid, dim3(32 * kTileWarps), smem, s, pdl, p);
+  return launch_kernel(kern, dim3(p.n_tiles), dim3(kTileThreads), 0, s, pdl, p);
 }
 
 // FFT variant of the FT convolution: the forms of two warps per item (default:
