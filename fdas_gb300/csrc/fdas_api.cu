@@ -16,6 +16,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "fdas_gb300.h"
@@ -45,6 +46,7 @@ constexpr int kCtrlStride = kCtrlStamp + 6;          // control words per buffer
 constexpr uint32_t kDefaultCapacity = 1u << 22;     // candidate records per buffer set
 constexpr uint32_t kMaxCapacity = 1u << 27;
 constexpr int kRecheckCap = 65536;
+constexpr uint32_t kHostRec = 4096;   // records mirrored in host memory (48 KB; ten times the 442 of a 2^18-bin search)
 constexpr int kNumEvents = 6;  // start, input, tiling, ftc, hsum, done
 
 struct BufferSet {
@@ -59,7 +61,14 @@ struct BufferSet {
   unsigned long long *d_key = nullptr;
   float *d_pwr = nullptr;
   unsigned *d_ctrl = nullptr;
-  unsigned *h_ctrl = nullptr;  // pinned mirror of d_ctrl
+  // results in pinned host memory, written by the selection's kernels: the control
+  // words, the fixed-size list and the first kHostRec records
+  unsigned *h_ctrl = nullptr;  // (the allocation's start; the batch owns its views')
+  uint32_t *h_cloc = nullptr;
+  float *h_cpwr = nullptr;
+  unsigned long long *h_key = nullptr;
+  float *h_pwr = nullptr;
+  bool results_on_host = false;  // the last harmonic summing was enqueued whole: they are the device's
   uint4 *d_rc = nullptr;
   unsigned *d_hist = nullptr;
   unsigned *d_ticket = nullptr;
@@ -440,6 +449,7 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
 
   if (hsum_smem_bytes(p) > 227 * 1024)
     return fail(h, FDAS_ERR_UNSUPPORTED, "harmonic summing staging exceeds shared memory (too many templates x planes)");
+  S.ctrl_valid = S.results_on_host = false;  // until the kernels that write them are enqueued
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl, 0, sizeof(unsigned) * kCtrlWords, S.stream));
   if (chain) p.stamp = stamp_at(S, 2);
   CK(h, launch_hsum(p, S.maps, S.stream, chain));
@@ -490,9 +500,17 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   f.ctrl = S.d_ctrl;
   f.host_ctrl = S.h_ctrl;
   f.n_ctrl = kCtrlStride;
-  f.host_loc = loc;
-  f.host_pwr = pwr;
+  // Host memory written by the kernels saves each retrieval its copies (four from
+  // pageable memory: 55 us for 442 records before, 20 after)
+  f.host_loc = S.h_cloc;
+  f.host_pwr = S.h_cpwr;
+  f.user_loc = loc;
+  f.user_pwr = pwr;
+  f.host_key = S.h_key;
+  f.host_rec_pwr = S.h_pwr;
+  f.n_host_rec = kHostRec;
   CK(h, launch_select(f, S.stream, chain));
+  S.results_on_host = true;
   CK(h, cudaEventRecord(S.ev[4], S.stream));
   S.ctrl_valid = true;
   return FDAS_OK;
@@ -577,6 +595,48 @@ void stage_times(const BufferSet &S, float *ms3) {
   ms3[0] = (float)(1e-6 * (double)(long long)(t[1] - t[0]));
   ms3[1] = (float)(1e-6 * (double)(long long)(t[2] - t[1]));
   ms3[2] = std::max(0.f, elapsed(S.ev[1], S.ev[4]) - ms3[0] - ms3[1]);
+}
+
+// Layout of a set's host memory from `base` (host_bytes() bytes, 16-byte aligned)
+size_t host_bytes(int planes, int per_plane) {
+  return ((sizeof(unsigned) * kCtrlStride + 15) & ~size_t(15)) + (sizeof(unsigned long long) + sizeof(float)) * kHostRec +
+         (((sizeof(uint32_t) + sizeof(float)) * (size_t)planes * per_plane + 15) & ~size_t(15));
+}
+void place_host(BufferSet &S, void *base, int planes, int per_plane) {
+  char *p = static_cast<char *>(base);
+  S.h_ctrl = reinterpret_cast<unsigned *>(p);
+  p += (sizeof(unsigned) * kCtrlStride + 15) & ~size_t(15);
+  S.h_key = reinterpret_cast<unsigned long long *>(p);
+  p += sizeof(unsigned long long) * kHostRec;
+  S.h_pwr = reinterpret_cast<float *>(p);
+  p += sizeof(float) * kHostRec;
+  S.h_cloc = reinterpret_cast<uint32_t *>(p);
+  S.h_cpwr = reinterpret_cast<float *>(S.h_cloc + (size_t)planes * per_plane);
+}
+
+// Control words and records of the last harmonic summing of a set whose stream
+// has completed: from host memory where they are there.
+fdas_status fetch_records(fdas_handle *h, BufferSet &S, unsigned *ctrl, bool records,
+                          std::vector<std::pair<unsigned long long, float>> *out) {
+  if (S.ctrl_valid) std::memcpy(ctrl, S.h_ctrl, sizeof(unsigned) * kCtrlWords);
+  else CK(h, cudaMemcpy(ctrl, S.d_ctrl, sizeof(unsigned) * kCtrlWords, cudaMemcpyDeviceToHost));
+  if (!records) return FDAS_OK;
+  const uint32_t stored = std::min(ctrl[kCtrlTotal], (unsigned)h->cap);
+  out->resize(stored);
+  const unsigned long long *keys = S.h_key;
+  const float *pwrs = S.h_pwr;
+  std::vector<unsigned long long> kv;
+  std::vector<float> pv;
+  if (stored && !(S.results_on_host && stored <= kHostRec)) {
+    kv.resize(stored);
+    pv.resize(stored);
+    CK(h, cudaMemcpy(kv.data(), S.d_key, sizeof(unsigned long long) * stored, cudaMemcpyDeviceToHost));
+    CK(h, cudaMemcpy(pv.data(), S.d_pwr, sizeof(float) * stored, cudaMemcpyDeviceToHost));
+    keys = kv.data();
+    pwrs = pv.data();
+  }
+  for (uint32_t i = 0; i < stored; ++i) (*out)[i] = {keys[i], pwrs[i]};
+  return FDAS_OK;
 }
 
 void free_set(BufferSet &S) {
@@ -757,12 +817,12 @@ fdas_status fdas_initialise_accelerator(const fdas_config *cfg_in, fdas_handle *
         (e = cudaMemset(S.d_hist, 0, sizeof(unsigned) * (size_t)h->P * kSelBuckets)) != cudaSuccess ||
         (e = cudaMemset(S.d_ticket, 0, sizeof(unsigned))) != cudaSuccess ||
         (e = cudaMemset(S.d_ctrl, 0, sizeof(unsigned) * kCtrlStride)) != cudaSuccess ||
-        (e = cudaHostAlloc((void **)&S.h_ctrl, sizeof(unsigned) * kCtrlStride, cudaHostAllocDefault)) !=
-            cudaSuccess ||
+        (e = cudaHostAlloc((void **)&S.h_ctrl, host_bytes(h->P, h->per_plane), cudaHostAllocDefault)) != cudaSuccess ||
         (e = cudaStreamCreateWithPriority(&S.stream, cudaStreamNonBlocking, h->cfg.stream_priority)) != cudaSuccess) {
       cuda_fail(h, e, "buffer set initialisation", __FILE__, __LINE__);
       return bail(FDAS_ERR_CUDA);
     }
+    place_host(S, S.h_ctrl, h->P, h->per_plane);
     std::memset(S.h_ctrl, 0, sizeof(unsigned) * kCtrlStride);
     if (make_hsum_maps(h, S) != FDAS_OK) return bail(FDAS_ERR_CUDA);
     for (auto &ev : S.ev) {
@@ -843,6 +903,7 @@ fdas_status fdas_reshape(fdas_handle *h, uint32_t n_frequency_bins, uint32_t tem
   h->cfg.n_planes = n_planes;
   for (auto &S : h->set) {
     S.have_input = S.fop_from_input = S.launched = S.ctrl_valid = S.series_spectrum = false;
+    S.results_on_host = false;
     S.ev_ftc_recorded = false;
     S.thresholds.clear();
     fdas_status st = make_hsum_maps(h, S);
@@ -1167,6 +1228,11 @@ fdas_status fdas_retrieve_candidates(fdas_handle *h, uint32_t *detection_locatio
   fdas_status st = sync_set(h, ab);
   if (st != FDAS_OK) return st;
   const size_t n = (size_t)h->P * h->per_plane;
+  if (h->set[ab].results_on_host) {
+    std::memcpy(detection_location, h->set[ab].h_cloc, sizeof(uint32_t) * n);
+    std::memcpy(detection_power, h->set[ab].h_cpwr, sizeof(float) * n);
+    return FDAS_OK;
+  }
   CK(h, cudaMemcpy(detection_location, h->set[ab].d_cloc, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
   CK(h, cudaMemcpy(detection_power, h->set[ab].d_cpwr, sizeof(float) * n, cudaMemcpyDeviceToHost));
   return FDAS_OK;
@@ -1182,7 +1248,8 @@ fdas_status fdas_retrieve_candidate_list(fdas_handle *h, fdas_candidate *out, ui
   if (st != FDAS_OK) return st;
   BufferSet &S = h->set[ab];
   unsigned ctrl[kCtrlWords];
-  CK(h, cudaMemcpy(ctrl, S.d_ctrl, sizeof(ctrl), cudaMemcpyDeviceToHost));
+  std::vector<std::pair<unsigned long long, float>> recs;
+  if ((st = fetch_records(h, S, ctrl, capacity > 0, &recs)) != FDAS_OK) return st;
   uint32_t total = 0;
   for (int pl = 0; pl < h->P; ++pl) total += ctrl[kCtrlCount + pl];
   const uint32_t stored = std::min(ctrl[kCtrlTotal], (unsigned)h->cap);
@@ -1191,24 +1258,16 @@ fdas_status fdas_retrieve_candidate_list(fdas_handle *h, fdas_candidate *out, ui
     if (n_dropped) *n_dropped = total - stored;
     return FDAS_OK;
   }
-  std::vector<unsigned long long> keys(stored);
-  std::vector<float> pwrs(stored);
-  if (stored) {
-    CK(h, cudaMemcpy(keys.data(), S.d_key, sizeof(unsigned long long) * stored, cudaMemcpyDeviceToHost));
-    CK(h, cudaMemcpy(pwrs.data(), S.d_pwr, sizeof(float) * stored, cudaMemcpyDeviceToHost));
-  }
   // (harmonic, template, bin) order, as hsum.py lists its detections
-  std::vector<uint32_t> idx(stored);
-  std::iota(idx.begin(), idx.end(), 0u);
-  std::sort(idx.begin(), idx.end(), [&](uint32_t a, uint32_t b) { return keys[a] < keys[b]; });
+  std::sort(recs.begin(), recs.end(), [](const auto &a, const auto &b) { return a.first < b.first; });
   const uint32_t n = std::min(stored, capacity);
   for (uint32_t i = 0; i < n; ++i) {
-    const unsigned long long k = keys[idx[i]];
+    const unsigned long long k = recs[i].first;
     fdas_candidate &c = out[i];
     c.harmonic = (uint32_t)(k >> 48) + 1;
     c.template_num = (int32_t)((k >> 32) & 0xffffu) - h->H;
     c.bin = (uint32_t)(k & 0xffffffffu);
-    c.power = pwrs[idx[i]];
+    c.power = recs[i].second;
   }
   if (n_total) *n_total = total;
   if (n_dropped) *n_dropped = total - stored;
@@ -1227,14 +1286,9 @@ fdas_status fdas_retrieve_candidates_ring(fdas_handle *h, uint32_t *detection_lo
   if (st != FDAS_OK) return st;
   BufferSet &S = h->set[ab];
   unsigned ctrl[kCtrlWords];
-  CK(h, cudaMemcpy(ctrl, S.d_ctrl, sizeof(ctrl), cudaMemcpyDeviceToHost));
-  const uint32_t stored = std::min(ctrl[kCtrlTotal], (unsigned)h->cap);
-  std::vector<unsigned long long> keys(stored);
-  std::vector<float> pwrs(stored);
-  if (stored) {
-    CK(h, cudaMemcpy(keys.data(), S.d_key, sizeof(unsigned long long) * stored, cudaMemcpyDeviceToHost));
-    CK(h, cudaMemcpy(pwrs.data(), S.d_pwr, sizeof(float) * stored, cudaMemcpyDeviceToHost));
-  }
+  std::vector<std::pair<unsigned long long, float>> recs;
+  if ((st = fetch_records(h, S, ctrl, true, &recs)) != FDAS_OK) return st;
+  const uint32_t stored = (uint32_t)recs.size();
   // FPGA geometry of the shipped design: groups of 4 templates, bundles of 2
   // bins, 64 slots of 8 lanes per plane (gen_info.h:47-54)
   constexpr int kGroup = 4, kBundle = 2, kSlots = 64, kLanes = 8;
@@ -1252,9 +1306,9 @@ fdas_status fdas_retrieve_candidates_ring(fdas_handle *h, uint32_t *detection_lo
   };
   std::vector<std::vector<Hit>> per_plane(h->P);
   for (uint32_t i = 0; i < stored; ++i) {
-    const int plane = (int)(keys[i] >> 48);
-    const int row = (int)((keys[i] >> 32) & 0xffffu);
-    const uint32_t bin = (uint32_t)(keys[i] & 0xffffffffu);
+    const int plane = (int)(recs[i].first >> 48);
+    const int row = (int)((recs[i].first >> 32) & 0xffffu);
+    const uint32_t bin = (uint32_t)(recs[i].first & 0xffffffffu);
     const int t = row - h->H;
     if ((which == FDAS_NEGATIVE_ACCELERATIONS && t > 0) || (which == FDAS_POSITIVE_ACCELERATIONS && t < 0)) continue;
     const int at = t < 0 ? -t : t;
@@ -1262,7 +1316,7 @@ fdas_status fdas_retrieve_candidates_ring(fdas_handle *h, uint32_t *detection_lo
     x.ev = ((unsigned long long)(at / kGroup) << 32) | (bin / kBundle);
     x.lane = (at % kGroup) * kBundle + (int)(bin % kBundle);
     x.loc = (((unsigned)plane & 7u) << 29) | (((unsigned)row & 0x7fu) << 22) | (bin & 0x3fffffu);
-    x.pwr = pwrs[i];
+    x.pwr = recs[i].second;
     per_plane[plane].push_back(x);
   }
   for (int pl = 0; pl < h->P; ++pl) {
@@ -1452,7 +1506,7 @@ struct fdas_batch {
   int *d_status = nullptr, *h_status = nullptr;
   unsigned long long *d_key = nullptr, *d_sel_key = nullptr;
   float *d_pwr = nullptr, *d_sel_pwr = nullptr, *d_cpwr = nullptr;
-  unsigned *d_ctrl = nullptr, *h_ctrl = nullptr, *d_hist = nullptr, *d_ticket = nullptr;
+  unsigned *d_ctrl = nullptr, *h_ctrl = nullptr /* all trials' host memory */, *d_hist = nullptr, *d_ticket = nullptr;
   uint4 *d_rc = nullptr;
   uint32_t *d_cloc = nullptr;
   std::vector<fdas_handle *> views;
@@ -1758,7 +1812,7 @@ fdas_status fdas_batch_create(const fdas_batch_config *cfg, const fdas_complex *
       (e = cudaMemset(b->d_hist, 0, sizeof(unsigned) * n * P * kSelBuckets)) != cudaSuccess ||
       (e = cudaMemset(b->d_ticket, 0, sizeof(unsigned) * n)) != cudaSuccess ||
       (e = cudaMemset(b->d_ctrl, 0, sizeof(unsigned) * n * kCtrlStride)) != cudaSuccess ||
-      (e = cudaHostAlloc((void **)&b->h_ctrl, sizeof(unsigned) * n * kCtrlStride, cudaHostAllocDefault)) != cudaSuccess ||
+      (e = cudaHostAlloc((void **)&b->h_ctrl, n * host_bytes(b->P, per_plane), cudaHostAllocDefault)) != cudaSuccess ||
       (e = cudaHostAlloc((void **)&b->h_status, sizeof(int), cudaHostAllocDefault)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&b->main, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaEventCreate(&b->t0)) != cudaSuccess || (e = cudaEventCreate(&b->t1)) != cudaSuccess) {
@@ -1827,7 +1881,8 @@ fdas_status fdas_batch_create(const fdas_batch_config *cfg, const fdas_complex *
     S.d_key = b->d_key + (size_t)i * cap;
     S.d_pwr = b->d_pwr + (size_t)i * cap;
     S.d_ctrl = b->d_ctrl + (size_t)i * kCtrlStride;
-    S.h_ctrl = b->h_ctrl + (size_t)i * kCtrlStride;
+    place_host(S, reinterpret_cast<char *>(b->h_ctrl) + (size_t)i * host_bytes(b->P, per_plane), b->P, per_plane);
+    std::memset(S.h_ctrl, 0, sizeof(unsigned) * kCtrlStride);
     S.d_rc = b->d_rc + (size_t)i * kBatchRecheckCap;
     S.d_hist = b->d_hist + (size_t)i * P * kSelBuckets;
     S.d_ticket = b->d_ticket + i;

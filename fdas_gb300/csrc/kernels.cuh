@@ -218,8 +218,13 @@ struct SelectParams {
   float *sel_pwr;
   uint32_t *compat_loc;   // [plane][per_plane]
   float *compat_pwr;
-  uint32_t *host_loc = nullptr;  // the list once more, in pinned host memory
-  float *host_pwr = nullptr;
+  uint32_t *host_loc;     // the list once more, in the set's pinned host memory
+  float *host_pwr;
+  uint32_t *user_loc;     // and in the caller's, where that is pinned too (or null)
+  float *user_pwr;
+  unsigned long long *host_key;  // the first n_host_rec records, in pinned host memory
+  float *host_rec_pwr;
+  unsigned n_host_rec;
   uint32_t invalid_location;
   int *status;
   const unsigned *ctrl;   // n_ctrl control words, copied to pinned host memory at the end

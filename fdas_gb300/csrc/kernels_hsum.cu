@@ -1019,6 +1019,10 @@ __global__ void __launch_bounds__(256) select_gather_kernel(SelectParams p) {
       const unsigned long long key = k[u];
       const int plane = (int)(key >> 48);
       const float pw = w[u];
+      if (const unsigned i = base + u * stride; i < p.n_host_rec) {
+        p.host_key[i] = key;
+        p.host_rec_pwr[i] = pw;
+      }
       const int sb = sb_of[plane];
       const int b = pwr_bucket(pw);
       int list = -1;
@@ -1083,13 +1087,17 @@ __global__ void __launch_bounds__(1024) select_finalize_kernel(SelectParams p) {
   }
   __syncthreads();
   const int kept = keep_a + c;
-  uint32_t *cl = p.compat_loc + (size_t)plane * K, *hl = p.host_loc ? p.host_loc + (size_t)plane * K : nullptr;
-  float *cp = p.compat_pwr + (size_t)plane * K, *hp = p.host_pwr ? p.host_pwr + (size_t)plane * K : nullptr;
+  uint32_t *cl = p.compat_loc + (size_t)plane * K, *hl = p.host_loc + (size_t)plane * K,
+           *ul = p.user_loc ? p.user_loc + (size_t)plane * K : nullptr;
+  float *cp = p.compat_pwr + (size_t)plane * K, *hp = p.host_pwr + (size_t)plane * K,
+        *up = p.user_pwr ? p.user_pwr + (size_t)plane * K : nullptr;
   auto put = [&](int at, uint32_t loc, float pwr) {
     cl[at] = loc;
     cp[at] = pwr;
-    if (hl) hl[at] = loc;
-    if (hp) hp[at] = pwr;
+    hl[at] = loc;
+    hp[at] = pwr;
+    if (ul) ul[at] = loc;
+    if (up) up[at] = pwr;
   };
   // the control words are final: the kernels before have ended
   if (blockIdx.x == 0 && blockIdx.y == 0)
