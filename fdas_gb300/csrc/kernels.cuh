@@ -267,7 +267,7 @@ struct SeriesPass {
   int R, m, ns;
   int unit;               // 2N / (ns R): table steps per twiddle exponent
   int B, log_b;
-  int n_steps;
+  int n_steps, threads;
   int radix[8];
 };
 constexpr int kTwFine = 2048;  // entries of the fine twiddle table

@@ -50,3 +50,15 @@ def test_after_reshape():
         out = np.zeros(m, dtype=np.complex64)
         assert p.series_to_spectrum(s, FDAS.A, scale=1.0, spectrum=out), p.last_error
         check(out, s, m)
+
+
+# every step size (2 to 10, 12, 14 to 16) first, in between and last, ragged last columns,
+# and both sides of the two-pass range
+@pytest.mark.parametrize("n", [4, 7, 9, 10, 12, 14, 15, 36, 81, 90, 196, 210, 225, 343, 1890, 30870, 50625, 63504, 100000,
+                               157464, 262144, 540225, 655360, 656100, 1048576, 1049760])
+def test_step_sizes(n):
+    s = np.random.default_rng(n).standard_normal(2 * n).astype(np.float32)
+    p = make_pipeline(n, log=io.StringIO(), n_templates=3)
+    out = np.zeros(n, dtype=np.complex64)
+    assert p.series_to_spectrum(s, FDAS.A, scale=1.0, spectrum=out), p.last_error
+    check(out, s, n)
