@@ -519,19 +519,34 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
 // The candidate list of a search goes into the caller's arrays by the selection's
 // last kernel where they are pinned (two copies less at the end of a search), else
 // by copies.
-bool pinned(const void *ptr) {
+// (One range of pinned memory holds the whole array, and it is aligned for stores.)
+bool pinned(const void *ptr, size_t bytes, size_t align) {
   cudaPointerAttributes at{};
-  if (!ptr || cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+  if (!ptr || reinterpret_cast<uintptr_t>(ptr) % align) return false;
+  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return at.type == cudaMemoryTypeHost && at.devicePointer == ptr;
+  if (at.type != cudaMemoryTypeHost || at.devicePointer != ptr) return false;
+  static const auto attribute = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &q);
+    if (e != cudaSuccess) cudaGetLastError();
+    return reinterpret_cast<decltype(&cuPointerGetAttribute)>(e == cudaSuccess && q == cudaDriverEntryPointSuccess ? fn
+                                                                                                                : nullptr);
+  }();
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  const CUdeviceptr p = reinterpret_cast<CUdeviceptr>(ptr);
+  return attribute && attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) == CUDA_SUCCESS &&
+         attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) == CUDA_SUCCESS && start <= p && p - start + bytes <= size;
 }
 fdas_status enqueue_hsum_download(fdas_handle *h, int ab, const float *thr, fdas_fop_part which, bool chain, uint32_t *loc,
                                   float *pwr) {
   BufferSet &S = h->set[ab];
   const size_t n = (size_t)h->P * h->per_plane;
-  const bool direct = pinned(loc) && pinned(loc + n - 1) && pinned(pwr) && pinned(pwr + n - 1);
+  const bool direct = pinned(loc, sizeof(uint32_t) * n, alignof(uint32_t)) && pinned(pwr, sizeof(float) * n, alignof(float));
   fdas_status st = enqueue_hsum(h, ab, thr, which, chain, direct ? loc : nullptr, direct ? pwr : nullptr);
   if (st != FDAS_OK) return st;
   if (loc && !direct) CK(h, cudaMemcpyAsync(loc, S.d_cloc, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, S.stream));
@@ -1077,8 +1092,9 @@ fdas_status fdas_series_to_spectrum(fdas_handle *h, const float *samples, uint64
   p.tw = h->d_series_tw;
   p.n = h->N;
   p.scale = scale;
+  p.host = pinned(spectrum, sizeof(float2) * (size_t)h->N, alignof(float2)) ? reinterpret_cast<float2 *>(spectrum) : nullptr;
   CK(h, launch_series_spectrum(p, S.stream));
-  if (spectrum)
+  if (spectrum && !p.host)
     CK(h, cudaMemcpyAsync(spectrum, S.d_input, sizeof(float2) * (size_t)h->N, cudaMemcpyDeviceToHost, S.stream));
   CK(h, cudaStreamSynchronize(S.stream));
   S.series_spectrum = true;

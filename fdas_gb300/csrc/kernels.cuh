@@ -256,6 +256,7 @@ struct TapsParams {
 struct SeriesParams {
   const float2 *samples;  // the 2N samples as N complex values (p.z, or the caller's device memory: only read)
   float2 *z;              // N complex: the N-bin spectrum on exit
+  float2 *host;           // and once more in pinned host memory, or null
   float2 *scratch;        // N complex
   const float4 *tw;       // series_twiddle_count(n) entries
   int n;                  // N

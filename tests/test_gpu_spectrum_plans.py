@@ -62,3 +62,23 @@ def test_step_sizes(n):
     out = np.zeros(n, dtype=np.complex64)
     assert p.series_to_spectrum(s, FDAS.A, scale=1.0, spectrum=out), p.last_error
     check(out, s, n)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 77 * 25 * 4 // 11, 4096, 30870])
+def test_spectrum_into_pinned_memory(n):
+    """The last kernel writes a pinned array itself, others are copied to: the same spectrum,
+    and nothing next to it."""
+    from fdas_gb300.fdas import PinnedArray
+    s = np.random.default_rng(n).standard_normal(2 * n).astype(np.float32)
+    p = make_pipeline(n, log=io.StringIO(), n_templates=3)
+    want = np.zeros(n, dtype=np.complex64)
+    assert p.series_to_spectrum(s, FDAS.A, scale=1.0, spectrum=want), p.last_error
+    keep = PinnedArray((n + 2,), np.complex64)
+    keep.array[:] = 7
+    assert p.series_to_spectrum(s, FDAS.B, scale=1.0, spectrum=keep.array[1:n + 1]), p.last_error
+    assert np.array_equal(keep.array[1:n + 1], want) and keep.array[0] == 7 and keep.array[n + 1] == 7
+    raw = PinnedArray((8 * n + 8,), np.uint8)
+    shifted = raw.array[4:8 * n + 4].view(np.complex64)  # not aligned for whole stores
+    assert shifted.ctypes.data % 8 == 4
+    assert p.series_to_spectrum(s, FDAS.A, scale=1.0, spectrum=shifted), p.last_error
+    assert np.array_equal(shifted, want)
