@@ -512,7 +512,7 @@ __host__ __device__ constexpr int rev3(int k) { return ((k & 1) << 2) | (k & 2) 
 // x[i] -> (-1)^popcount(k) sum_i x[i] z^i e^(2 pi i i k / 8) at x[rev3(k)].
 // LAST: the transform's last DFT8, where a signal's peak and its weak neighbours
 // part: the outputs of its last two stages are not taken from one another (8 us of
-// 308 at 2^21 bins x 85 rows; in every stage of both DFT8: 32 us).
+// 303 at 2^21 bins x 85 rows; in every stage of both DFT8: 32 us).
 template <bool LAST>
 __device__ __forceinline__ void twisted_dft8(float2 *x, const TwistedTw &t) {
   bfly(x[0], x[4], t.t4);
@@ -630,7 +630,8 @@ __device__ __forceinline__ void twisted_store(const float2 *v, float2 *buf, int 
 // Pass 2: put(r, d2, |y[m + 32 (4 g + r) + 256 d2]|^2) for the thread's 32
 // outputs.  ``tw.issue(k, t)`` starts the load of a set of twiddles into t
 // (k = 0: the first DFT8, 1 + r: slot r of the second) and ``tw.wait(t)``
-// completes it; ``after_read`` runs once the pair buffer has been read.
+// completes it; Tw::kEarly: slot 0's set is fetched before the first DFT8s, not
+// after them; ``after_read`` runs once the pair buffer has been read.
 template <typename Tw, typename Hook, typename Put>
 __device__ __forceinline__ void twisted_pass2(const float2 *buf, const Tw &tw, int tp, Hook after_read, Put put) {
   const int l = tp & 31, m = 16 * (tp >> 5) + (l & 15), g = l >> 4;
@@ -647,8 +648,9 @@ __device__ __forceinline__ void twisted_pass2(const float2 *buf, const Tw &tw, i
   });
   tw.wait(t);
   after_read();
+  if constexpr (Tw::kEarly) tw.issue(1, tn);
   sfor<4>([&](auto Q) { twisted_dft8<false>(u + 8 * decltype(Q)::value, t); });
-  tw.issue(1, t);
+  if constexpr (!Tw::kEarly) tw.issue(1, tn);
   sfor<4>([&](auto Q) {
     constexpr int q = decltype(Q)::value;
     sfor<4>([&](auto R) {
@@ -657,7 +659,8 @@ __device__ __forceinline__ void twisted_pass2(const float2 *buf, const Tw &tw, i
       x.y = __shfl_xor_sync(0xffffffffu, x.y, 16);
     });
   });
-  tw.wait(t);
+  tw.wait(tn);
+  t = tn;
   sfor<4>([&](auto R) {
     constexpr int r = decltype(R)::value;
     if constexpr (r < 3) tw.issue(2 + r, tn);

@@ -383,8 +383,8 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
 // ---------------------------------------------------------------------------
 // Group form, the FT convolution wherever it has the SMs for itself: 8 warp
 // pairs per CTA, one CTA per SM, each pair with one tile of a group of
-// consecutive tiles, all of them on the same template row at about the same time.  The template rows pass through a ring of shared-memory slots,
-// one 16 KB TMA copy for all pairs of the CTA.  The pair's tile spectrum and
+// consecutive tiles, all of them on the same template row at about the same time.
+// The template rows pass through a ring of shared-memory slots, one 16 KB TMA copy for all pairs of the CTA.  The pair's tile spectrum and
 // its twiddles stay in tensor memory over the rows, used as 128 words of
 // private storage per thread (32 lanes x 128 columns per warp): registers hold
 // one transform only, and neither passes through L1 / shared memory again.
@@ -394,10 +394,12 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
 // Bound by the shared-memory pipe and the FMA pipe about alike (2^19 bins x 85
 // rows: 64% and 63% busy, ~600 wavefronts and ~550 FMA-pipe clocks per item of
 // ~880 clocks); the pair form below moves ~960 wavefronts and 680 clocks per
-// item.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 308 / 82 / 11.3 us
+// item.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 303 / 81 / 11.1 us
 // against 432 / 118 / 19.4 us of the pair form.  The same with 6 pairs and the
 // tile in registers (168 a thread) took 361 us, 4 pairs of two rows each 488 us;
-// the twiddle products all packed 336 us, all scalar 345 us.
+// the twiddle products all packed 336 us, all scalar 345 us; pass 2 with the real
+// and imaginary parts of two DFT8s side by side (all packed, but re-paired after the
+// exchange) 322, an mbarrier in place of the barrier before the exchange 321.
 constexpr int kGroupPairs = 8;
 constexpr int kGroupRing = 5;  // what 227 KB hold beside eight pair buffers
 constexpr int kGroupSmem = (kGroupRing * 2 * kTile + kGroupPairs * kEx2Floats) * (int)sizeof(float);
@@ -466,7 +468,11 @@ __device__ __forceinline__ void tm_st_tw(uint32_t addr, const TwistedTw &t) {
 }
 __device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// The first set of the second DFT8 fetched while the DFT8s before it run: 308 -> 303 us
+// at 2^21 bins x 85 rows; the batched form (24 trials 4652 us) took 4664 with it.
+template <bool BATCH>
 struct TmemTwiddles {
+  static constexpr bool kEarly = !BATCH;
   uint32_t base;
   __device__ __forceinline__ void issue(int k, TwistedTw &t) const { tm_ld_tw(base + kTmTw + 8 * k, t); }
   __device__ __forceinline__ void wait(TwistedTw &t) const {
@@ -549,7 +555,7 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
     tm_st16(tm + kTmTile + 32, v + 16);
     tm_wait_st();
   }
-  const TmemTwiddles tw{tm};
+  const TmemTwiddles<BATCH> tw{tm};
 
   bool active = false, fresh = true, inner = false;
   int lo = 0, hi = 0;
