@@ -91,6 +91,7 @@ __device__ __forceinline__ int batch_trial_of(const BatchTrial *tr, int n, long 
 
 struct TileParams {
   const float2 *input;    // N spectrum bins
+  float2 *copy = nullptr; // N bins: where the input is host memory, its copy for the later kernels
   int n_bins;
   int n_tiles;
   int overlap;            // O

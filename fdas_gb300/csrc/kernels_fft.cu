@@ -25,7 +25,8 @@ constexpr int kWarpsPerCta = 8;
 // tile's padding) read as zero -- tile_input.cl.mako:42-94 / ft_conv.py:165-180.
 constexpr int kTileThreads = 128;
 constexpr int kTilePitch = 129;  // odd: the column reads of the first exchange meet no bank twice
-template <bool BATCH>
+// HOST: the input is pinned host memory, and its copy is left at p.copy.
+template <bool BATCH, bool HOST>
 __global__ void __launch_bounds__(kTileThreads, 8) tile_fft_kernel(TileParams p) {
   __shared__ float2 ex[16 * kTilePitch];
   const int t = threadIdx.x;
@@ -58,6 +59,12 @@ __global__ void __launch_bounds__(kTileThreads, 8) tile_fft_kernel(TileParams p)
     const long long b = start + 128 * n1;
     v[n1] = (b >= 0 && b < n_bins) ? input[b] : make_float2(0.f, 0.f);
   });
+  if constexpr (HOST)  // the bins past the overlap are this tile's own
+    sfor<16>([&](auto N1) {
+      constexpr int n1 = decltype(N1)::value;
+      const long long b = start + 128 * n1;
+      if (t + 128 * n1 >= p.overlap && b < n_bins) p.copy[b] = v[n1];
+    });
   // (the table holds w^j = e^(+2 pi i j / 2048); conjugated here)
   auto conj_mul = [](float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.y, b.x, -a.x * b.y));
@@ -721,7 +728,7 @@ int current_sm_count() {
 static int ex_smem_bytes() { return kWarpsPerCta * kExFloats * (int)sizeof(float); }
 
 cudaError_t launch_tile_fft(const TileParams &p, cudaStream_t s, bool pdl) {
-  auto kern = p.trials ? tile_fft_kernel<true> : tile_fft_kernel<false>;
+  auto kern = p.trials ? tile_fft_kernel<true, false> : p.copy ? tile_fft_kernel<false, true> : tile_fft_kernel<false, false>;
   return launch_kernel(kern, dim3(p.n_tiles), dim3(kTileThreads), 0, s, pdl, p);
 }
 
