@@ -485,6 +485,7 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
     r.input = S.cur_input;
     r.n_bins = h->N;
     r.half = H;
+    r.n_planes = P;
     r.taps = reinterpret_cast<const float4 *>(S.d_taps + (size_t)h->row0 * h->tap_pitch);
     r.tap_len = S.d_taplen + h->row0;
     r.tap_pitch = h->tap_pitch;

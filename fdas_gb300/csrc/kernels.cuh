@@ -184,6 +184,7 @@ struct HsumMaps {
 struct RecheckParams {
   const float2 *input;    // the spectrum the FOP was computed from
   int n_bins;
+  int n_planes;
   int half;
   const float4 *taps;     // n_templates x tap_pitch time-domain taps as float pairs
                           // (re hi, im hi, re lo, im lo): tap = hi + lo to 2^-48

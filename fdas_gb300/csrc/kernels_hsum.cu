@@ -829,9 +829,11 @@ __device__ __forceinline__ void df_add_prod(float &s, float &t, float a, float b
 // double-float arithmetic (about 2^-44 relative), then in FP64 across the
 // lanes; warp 0 sums the planes in order j = 1..k (hsum.py:95-120) in FP64
 // and compares with the threshold.  A noise-like search has a handful of entries, so
-// the launch lasts as long as one of them: a warp for each of 16 planes (8 warps took
-// two turns: harmonic-summing stage of 2^20 bins x 16 planes 134.3 -> 129.5 us, of
-// 300007 bins x 43 rows 52.0 -> 51.1; 8 planes gain 0.5 from the fewer CTAs).
+// the launch lasts as long as one of them: a warp for each plane, 16 above 8 planes
+// (8 warps took two turns: harmonic-summing stage of 2^20 bins x 16 planes 134.3 ->
+// 129.5 us, of 300007 bins x 43 rows 52.0 -> 51.1).  Up to 8 planes half of those
+// would be idle, and an SM holds three CTAs of 8 warps but one of 16: 413 entries
+// (2^21 bins, three strong signals) 9.0 against 14.6 us.
 __global__ void __launch_bounds__(512) recheck_kernel(RecheckParams p) {
   __shared__ double cell[kMaxPlanes];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1179,7 +1181,8 @@ cudaError_t launch_split_taps(double2 *taps, long long n, cudaStream_t s) {
 }
 
 cudaError_t launch_recheck(const RecheckParams &p, cudaStream_t s, bool pdl) {
-  return launch_kernel(recheck_kernel, dim3(2 * current_sm_count()), dim3(32 * 16), 0, s, pdl, p);
+  const int warps = p.n_planes <= 8 ? 8 : 16;
+  return launch_kernel(recheck_kernel, dim3(32 / warps * current_sm_count()), dim3(32 * warps), 0, s, pdl, p);
 }
 
 cudaError_t launch_select(const SelectParams &p, cudaStream_t s, bool pdl) {
