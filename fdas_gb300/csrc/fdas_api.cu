@@ -402,7 +402,7 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which, bool chain)
   // A search whose spectrum was copied from host memory starts its FT
   // convolution only once the other set's harmonic-summing kernel has ended.
   // Otherwise that harmonic summing finds every SM held by this FT convolution
-  // (two CTAs of 128 registers x 256 threads fill an SM's register file), both
+  // (a CTA of 512 threads x 120 registers fills an SM's register file), both
   // searches end together, and with launch(A) / wait(B) the next launch -- its
   // 16 MB copy and tiling -- starts on an empty GPU every second search.
   // Device-resident searches queued ahead keep the unordered form, where the

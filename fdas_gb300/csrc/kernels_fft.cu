@@ -399,9 +399,8 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
 // grid, so every CTA has the same number of steps to within one whatever the
 // number of tiles.
 // Bound by the shared-memory pipe and the FMA pipe about alike (2^19 bins x 85
-// rows: 64% and 63% busy, ~600 wavefronts and ~550 FMA-pipe clocks per item of
-// ~880 clocks); the pair form below moves ~960 wavefronts and 680 clocks per
-// item.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 303 / 81 / 11.1 us
+// rows: 67% and 65% busy, math-pipe throttling first among the stalls, 475
+// shared-memory wavefronts per item); the pair form below has 654 and its L1TEX pipe 78% busy.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 303 / 81 / 11.1 us
 // against 432 / 118 / 19.4 us of the pair form.  The same with 6 pairs and the
 // tile in registers (168 a thread) took 361 us, 4 pairs of two rows each 488 us;
 // the twiddle products all packed 336 us, all scalar 345 us; pass 2 with the real

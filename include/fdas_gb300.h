@@ -280,7 +280,7 @@ fdas_status fdas_set_wait_timeout(fdas_handle *h, int64_t ns);
 
 /* Test hooks for the timeout paths (no counterpart in the reference).  With
  * FDAS_INJECT_FTC_STALL set, the FT convolution of later searches announces
- * each warp pair's first template copy on its barrier but never issues it, so
+ * each CTA's first template copy on its barrier but never issues it, so
  * that wait cannot complete and runs out after the bound of
  * fdas_set_wait_timeout: the search stops with the FT-convolution timeout bit
  * and fdas_wait returns FDAS_ERR_TIMEOUT.  FDAS_INJECT_HSUM_STALL does the
