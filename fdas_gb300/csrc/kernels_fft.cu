@@ -391,17 +391,19 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
 // Group form, the FT convolution wherever it has the SMs for itself: 8 warp
 // pairs per CTA, one CTA per SM, each pair with one tile of a group of
 // consecutive tiles, all of them on the same template row at about the same time.
-// The template rows pass through a ring of shared-memory slots, one 16 KB TMA copy for all pairs of the CTA.  The pair's tile spectrum and
-// its twiddles stay in tensor memory over the rows, used as 128 words of
-// private storage per thread (32 lanes x 128 columns per warp): registers hold
-// one transform only, and neither passes through L1 / shared memory again.
+// The template rows pass through a ring of shared-memory slots, one 16 KB TMA
+// copy for all pairs of the CTA.  The pair's tile spectrum and its twiddles stay
+// in tensor memory over the rows, used as 128 words of private storage per thread
+// (32 lanes x 128 columns per warp): registers hold one transform only, and
+// neither passes through L1 / shared memory again.
 // Work: the steps (group, row) in row-major order are split evenly over the
 // grid, so every CTA has the same number of steps to within one whatever the
 // number of tiles.
 // Bound by the shared-memory pipe and the FMA pipe about alike (2^19 bins x 85
 // rows: 67% and 65% busy, math-pipe throttling first among the stalls, 475
-// shared-memory wavefronts per item); the pair form below has 654 and its L1TEX pipe 78% busy.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 303 / 81 / 11.1 us
-// against 432 / 118 / 19.4 us of the pair form.  The same with 6 pairs and the
+// shared-memory wavefronts per item); the pair form below has 654 and its L1TEX
+// pipe 78% busy.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 303 / 81 /
+// 11.1 us against 432 / 118 / 19.4 us of the pair form.  The same with 6 pairs and the
 // tile in registers (168 a thread) took 361 us, 4 pairs of two rows each 488 us;
 // the twiddle products all packed 336 us, all scalar 345 us; pass 2 with the real
 // and imaginary parts of two DFT8s side by side (all packed, but re-paired after the
