@@ -100,6 +100,9 @@ struct BufferSet {
   bool ev_hsum_recorded = false;
   bool input_from_host = false;   // the current spectrum was copied in from host memory
   const float2 *host_input = nullptr;  // read by the next tiling instead of d_input, which it fills
+  // events that end the input copy and the harmonic summing: the launch's first and
+  // last where nothing is copied (an event in between delays the kernels by 2 us)
+  int ev_in = 1, ev_hs = 4;
   bool stamped = false;           // the last search was enqueued in one go: ev[2], ev[3] are times in the control words
   bool used = false;              // a search or stage ran on this set
 };
@@ -316,7 +319,8 @@ fdas_status enqueue_input(fdas_handle *h, int ab, const fdas_complex *input, boo
     S.series_spectrum = false;
     S.input_from_host = true;
   }
-  CK(h, cudaEventRecord(S.ev[1], S.stream));
+  S.ev_in = h->cfg.sync_pipeline || (S.input_from_host && !S.host_input) ? 1 : 0;
+  if (S.ev_in == 1) CK(h, cudaEventRecord(S.ev[1], S.stream));
   S.have_input = true;
   return FDAS_OK;
 }
@@ -420,7 +424,7 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which, bool chain)
 }
 
 fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_part which, bool chain,
-                         uint32_t *loc = nullptr, float *pwr = nullptr) {
+                         uint32_t *loc = nullptr, float *pwr = nullptr, bool end_event = true) {
   BufferSet &S = h->set[ab];
   const float *thr = thr_in;
   if (!thr) {
@@ -534,7 +538,8 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   f.n_host_rec = kHostRec;
   CK(h, launch_select(f, S.stream, chain));
   S.results_on_host = true;
-  CK(h, cudaEventRecord(S.ev[4], S.stream));
+  S.ev_hs = end_event ? 4 : 5;
+  if (end_event) CK(h, cudaEventRecord(S.ev[4], S.stream));
   S.ctrl_valid = true;
   return FDAS_OK;
 }
@@ -570,7 +575,8 @@ fdas_status enqueue_hsum_download(fdas_handle *h, int ab, const float *thr, fdas
   BufferSet &S = h->set[ab];
   const size_t n = (size_t)h->P * h->per_plane;
   const bool direct = pinned(loc, sizeof(uint32_t) * n, alignof(uint32_t)) && pinned(pwr, sizeof(float) * n, alignof(float));
-  fdas_status st = enqueue_hsum(h, ab, thr, which, chain, direct ? loc : nullptr, direct ? pwr : nullptr);
+  fdas_status st = enqueue_hsum(h, ab, thr, which, chain, direct ? loc : nullptr, direct ? pwr : nullptr,
+                                !direct && (loc || pwr));
   if (st != FDAS_OK) return st;
   if (loc && !direct) CK(h, cudaMemcpyAsync(loc, S.d_cloc, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, S.stream));
   if (pwr && !direct) CK(h, cudaMemcpyAsync(pwr, S.d_cpwr, sizeof(float) * n, cudaMemcpyDeviceToHost, S.stream));
@@ -625,14 +631,15 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
 // ms of tiling, FT convolution and harmonic summing of a completed search
 void stage_times(const BufferSet &S, float *ms3) {
   if (!S.stamped) {
-    for (int i = 0; i < 3; ++i) ms3[i] = elapsed(S.ev[1 + i], S.ev[2 + i]);
+    const int at[4] = {S.ev_in, 2, 3, S.ev_hs};
+    for (int i = 0; i < 3; ++i) ms3[i] = elapsed(S.ev[at[i]], S.ev[at[i + 1]]);
     return;
   }
   unsigned long long t[3];
   std::memcpy(t, S.h_ctrl + kCtrlStamp, sizeof(t));
   ms3[0] = (float)(1e-6 * (double)(long long)(t[1] - t[0]));
   ms3[1] = (float)(1e-6 * (double)(long long)(t[2] - t[1]));
-  ms3[2] = std::max(0.f, elapsed(S.ev[1], S.ev[4]) - ms3[0] - ms3[1]);
+  ms3[2] = std::max(0.f, elapsed(S.ev[S.ev_in], S.ev[S.ev_hs]) - ms3[0] - ms3[1]);
 }
 
 // Layout of a set's host memory from `base` (host_bytes() bytes, 16-byte aligned)
@@ -1044,7 +1051,7 @@ fdas_status fdas_perform_input_tiling(fdas_handle *h, const fdas_complex *input,
   if (st != FDAS_OK) return st;
   if ((st = enqueue_tiling(h, ab, false)) != FDAS_OK) return st;
   if ((st = sync_set(h, ab)) != FDAS_OK) return st;
-  logf(h, "[INFO] Preparation duration: %.3f ms", elapsed(h->set[ab].ev[1], h->set[ab].ev[2]));
+  logf(h, "[INFO] Preparation duration: %.3f ms", elapsed(h->set[ab].ev[h->set[ab].ev_in], h->set[ab].ev[2]));
   return FDAS_OK;
 }
 
@@ -1076,7 +1083,7 @@ fdas_status fdas_perform_harmonic_summing(fdas_handle *h, const float *threshold
   fdas_status st = enqueue_hsum(h, ab, thresholds, which, false);
   if (st != FDAS_OK) return st;
   if ((st = sync_set(h, ab)) != FDAS_OK) return st;
-  logf(h, "[INFO] Harmonic summing duration: %.3f ms", elapsed(S.ev[3], S.ev[4]));
+  logf(h, "[INFO] Harmonic summing duration: %.3f ms", elapsed(S.ev[3], S.ev[S.ev_hs]));
   return FDAS_OK;
 }
 
@@ -1386,11 +1393,11 @@ fdas_status fdas_get_stage_times(fdas_handle *h, fdas_buffer_set ab, float *ms6)
   CK(h, cudaEventSynchronize(S.ev[5]));
   float st[3];
   stage_times(S, st);
-  ms6[0] = elapsed(S.ev[0], S.ev[1]);
+  ms6[0] = elapsed(S.ev[0], S.ev[S.ev_in]);
   ms6[1] = st[0];
   ms6[2] = st[1];
   ms6[3] = st[2];
-  ms6[4] = elapsed(S.ev[4], S.ev[5]);
+  ms6[4] = elapsed(S.ev[S.ev_hs], S.ev[5]);
   ms6[5] = elapsed(S.ev[0], S.ev[5]);
   return FDAS_OK;
 }
@@ -1455,8 +1462,9 @@ void fdas_print_events(fdas_handle *h, fdas_buffer_set ab) {
   // convolution, harmonic summing and candidate transfer; each stage starts
   // where the one before it ends on the set's stream
   long long t[6];
+  const int at[6] = {0, S.ev_in, 2, 3, S.ev_hs, 5};
   for (int i = 0; i < 6; ++i)
-    if (!S.stamped || (i != 2 && i != 3)) t[i] = event_ns(h, S.ev[i]);
+    if (!S.stamped || (i != 2 && i != 3)) t[i] = event_ns(h, S.ev[at[i]]);
   if (S.stamped) {
     float st[3];
     stage_times(S, st);
