@@ -50,25 +50,6 @@ float2 *g_scratch_ptr[kMaxDevices] = {};
 float2 g_twiddle_host[kTile];
 bool g_twiddle_host_ready = false;
 
-// p4 position 4 s + j holds natural bin bitrev2(j) * 512 + s
-// (tmpl-gen.py:145-153); natural bin k therefore sits at p4 position
-// 4 (k mod 512) + bitrev2(k / 512).  Spectra are scaled by 2^-11 (the inverse
-// transform's 1/2048, exact in float) as the handle does at upload.
-__global__ void noalloc_templates_kernel(const float2 *__restrict__ src, float2 *__restrict__ dst, int n_templates,
-                                         int p4) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = blockIdx.y;
-  grid_release();
-  if (k >= kTile || r >= n_templates) return;
-  int q = k;
-  if (p4) {
-    const int b = k >> 9;
-    q = 4 * (k & 511) + (((b & 1) << 1) | ((b >> 1) & 1));
-  }
-  const float2 v = src[(size_t)r * kTile + q];
-  dst[(size_t)r * kTile + k] = make_float2(v.x * (1.0f / 2048.0f), v.y * (1.0f / 2048.0f));
-}
-
 // Address of this device's scratch; on the first call for a device (with that
 // device current) it is looked up and the twiddle table is written into it.
 fdas_status scratch_for_current_device(float2 **out) {
@@ -139,9 +120,10 @@ extern "C" fdas_status fdas_ft_convolution_noalloc(const fdas_complex *d_spectru
   int *status_word = reinterpret_cast<int *>(twiddle + kTwElems);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-  noalloc_templates_kernel<<<dim3(kTile / 256, n_templates), 256, 0, s>>>(
-      reinterpret_cast<const float2 *>(d_templates), tmpl, (int)n_templates, layout == FDAS_TEMPLATES_FFT_P4);
-  if (cudaGetLastError() != cudaSuccess) return FDAS_ERR_CUDA;
+  // the rows that this call's sign half uses
+  const int T = (int)n_templates, H = T / 2;
+  const int row_begin = which == FDAS_POSITIVE_ACCELERATIONS ? H : 0;
+  const int n_rows = which == FDAS_ALL_ACCELERATIONS ? T : H + 1;
 
   TileParams tp{};
   tp.input = reinterpret_cast<const float2 *>(d_spectrum);
@@ -151,15 +133,18 @@ extern "C" fdas_status fdas_ft_convolution_noalloc(const fdas_complex *d_spectru
   tp.payload = (int)payload;
   tp.tiles = tiles;
   tp.twiddle = twiddle;
-  // the kernels start on each other's tails; a capture gets plain launches
+  tp.tmpl_src = reinterpret_cast<const float2 *>(d_templates) + (size_t)row_begin * kTile;
+  tp.tmpl_dst = tmpl + (size_t)row_begin * kTile;
+  tp.n_tmpl = n_rows;
+  tp.tmpl_p4 = layout == FDAS_TEMPLATES_FFT_P4;
+  // the second kernel starts on the first one's tail; a capture gets plain launches
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   const bool pdl = cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-  if (launch_tile_fft(tp, s, pdl) != cudaSuccess) {
+  if (launch_tile_fft(tp, s) != cudaSuccess) {
     cudaGetLastError();
     return FDAS_ERR_CUDA;
   }
 
-  const int T = (int)n_templates, H = T / 2;
   FtcParams fp{};
   fp.tiles = tiles;
   fp.tmpl = tmpl;
@@ -169,9 +154,8 @@ extern "C" fdas_status fdas_ft_convolution_noalloc(const fdas_complex *d_spectru
   fp.n_tiles = (int)n_tiles;
   fp.overlap = (int)tile_overlap;
   fp.payload = (int)payload;
-  if (which == FDAS_NEGATIVE_ACCELERATIONS) { fp.row_begin = 0; fp.n_rows = H + 1; }
-  else if (which == FDAS_POSITIVE_ACCELERATIONS) { fp.row_begin = H; fp.n_rows = H + 1; }
-  else { fp.row_begin = 0; fp.n_rows = T; }
+  fp.row_begin = row_begin;
+  fp.n_rows = n_rows;
   fp.twiddle = twiddle;
   fp.status = d_status ? reinterpret_cast<int *>(d_status) : status_word;
   fp.timeout_ns = 2000000000LL;  // 2 s

@@ -100,6 +100,12 @@ struct TileParams {
   const float2 *twiddle;  // e^(+2 pi i j / 2048), j < 2048
   const BatchTrial *trials = nullptr;  // batched search: n_tiles spans all trials
   int n_trials = 0;
+  // template rows to bring into the kernels' form by CTAs of their own (the
+  // allocation-free call): natural order, scaled by 2^-11
+  const float2 *tmpl_src = nullptr;
+  float2 *tmpl_dst = nullptr;
+  int n_tmpl = 0;
+  int tmpl_p4 = 0;           // the source is in p4 order
   unsigned *zero = nullptr;  // words to zero before the following kernels run (a search's control words)
   int n_zero = 0;
   unsigned long long *stamp = nullptr;  // start time (stage times of a search enqueued in one go)
