@@ -21,6 +21,7 @@
 
 #include "fdas_gb300.h"
 #include "kernels.cuh"
+#include "pointers.cuh"
 
 using namespace fdas;
 
@@ -544,6 +545,24 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   return FDAS_OK;
 }
 
+// Start and size of the allocation around an address (size 0 where the driver does not say)
+void range_at(const void *ptr, uint64_t *start, uint64_t *size) {
+  static const auto attribute = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &q);
+    if (e != cudaSuccess) cudaGetLastError();
+    return reinterpret_cast<decltype(&cuPointerGetAttribute)>(e == cudaSuccess && q == cudaDriverEntryPointSuccess ? fn
+                                                                                                                : nullptr);
+  }();
+  CUdeviceptr at = 0;
+  size_t n = 0;
+  const CUdeviceptr p = reinterpret_cast<CUdeviceptr>(ptr);
+  const bool known = attribute && attribute(&at, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) == CUDA_SUCCESS &&
+                     attribute(&n, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) == CUDA_SUCCESS;
+  *start = at;
+  *size = known ? n : 0;
+}
 // The candidate list of a search goes into the caller's arrays by the selection's
 // last kernel where they are pinned (two copies less at the end of a search), else
 // by copies.
@@ -556,19 +575,21 @@ bool pinned(const void *ptr, size_t bytes, size_t align) {
     return false;
   }
   if (at.type != cudaMemoryTypeHost || at.devicePointer != ptr) return false;
-  static const auto attribute = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &q);
-    if (e != cudaSuccess) cudaGetLastError();
-    return reinterpret_cast<decltype(&cuPointerGetAttribute)>(e == cudaSuccess && q == cudaDriverEntryPointSuccess ? fn
-                                                                                                                : nullptr);
-  }();
-  CUdeviceptr start = 0;
-  size_t size = 0;
-  const CUdeviceptr p = reinterpret_cast<CUdeviceptr>(ptr);
-  return attribute && attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) == CUDA_SUCCESS &&
-         attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) == CUDA_SUCCESS && start <= p && p - start + bytes <= size;
+  uint64_t start, size;
+  range_at(ptr, &start, &size);
+  const uint64_t p = reinterpret_cast<uintptr_t>(ptr);
+  return start <= p && p - start + bytes <= size;
+}
+// (what the driver does not know, not even as host memory, is no device memory)
+MemoryAt memory_at(const void *ptr) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    cudaGetLastError();
+    return MemoryAt{};
+  }
+  MemoryAt m{at.type == cudaMemoryTypeDevice && at.devicePointer == ptr, at.device, 0, 0};
+  if (m.device) range_at(ptr, &m.start, &m.size);
+  return m;
 }
 fdas_status enqueue_hsum_download(fdas_handle *h, int ab, const float *thr, fdas_fop_part which, bool chain, uint32_t *loc,
                                   float *pwr) {
@@ -1111,9 +1132,11 @@ fdas_status fdas_series_to_spectrum(fdas_handle *h, const float *samples, uint64
     h->series_tw_n = h->N;
   }
   // device samples are read where they are (as pairs, so 8-byte aligned ones)
-  const bool in_place = samples_on_device && reinterpret_cast<uintptr_t>(samples) % sizeof(float2) == 0;
+  const size_t sample_bytes = sizeof(float) * 2 * (size_t)h->N;
+  const bool in_place = samples_on_device && readable_in_place(memory_at(samples), reinterpret_cast<uintptr_t>(samples),
+                                                               sample_bytes, sizeof(float2), h->cfg.device);
   if (!in_place)
-    CK(h, cudaMemcpyAsync(S.d_input, samples, sizeof(float) * 2 * (size_t)h->N,
+    CK(h, cudaMemcpyAsync(S.d_input, samples, sample_bytes,
                           samples_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, S.stream));
   SeriesParams p{};
   p.samples = in_place ? reinterpret_cast<const float2 *>(samples) : S.d_input;
