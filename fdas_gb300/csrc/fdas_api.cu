@@ -341,7 +341,7 @@ bool can_chain(const fdas_handle *h, int ab, const float *thr) {
   p.half = h->H;
   p.n_planes = h->P;
   hsum_geometry(h, p);
-  return !h->cfg.precision && S.have_templates && (thr || !S.thresholds.empty()) && hsum_smem_bytes(p) <= 227 * 1024;
+  return !h->cfg.precision && S.have_templates && (thr || !S.thresholds.empty()) && hsum_smem_bytes(p) <= kHsMaxSmem;
 }
 
 fdas_status enqueue_tiling(fdas_handle *h, int ab, bool chain) {
@@ -474,7 +474,7 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   p.status = reinterpret_cast<int *>(S.d_ctrl + kCtrlStatus);
   p.timeout_ns = h->wait_timeout_ns;
 
-  if (hsum_smem_bytes(p) > 227 * 1024)
+  if (hsum_smem_bytes(p) > kHsMaxSmem)
     return fail(h, FDAS_ERR_UNSUPPORTED, "harmonic summing staging exceeds shared memory (too many templates x planes)");
   S.ctrl_valid = S.results_on_host = false;  // until the kernels that write them are enqueued
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl, 0, sizeof(unsigned) * kCtrlWords, S.stream));

@@ -50,6 +50,15 @@ __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.la
 __device__ __forceinline__ void stamp(unsigned long long *at) {
   if (at && blockIdx.x == 0 && threadIdx.x == 0) asm volatile("mov.u64 %0, %globaltimer;" : "=l"(*at));
 }
+// Lets a kernel be launched with up to `bytes` of dynamic shared memory.  The limit is
+// one per kernel and device, shared by every handle and thread: `bytes` is the most that
+// any launch of the kernel takes, never this launch's own, or a thread with a smaller
+// launch would lower it between another's call and its launch (which then fails: 18 of
+// 2000 series FFTs of 2^20 points beside a thread with 4096).
+template <typename Kernel>
+cudaError_t allow_smem(Kernel kern, int bytes) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
 template <typename Kernel, typename... Args>
 cudaError_t launch_kernel(Kernel kern, dim3 grid, dim3 block, int smem, cudaStream_t s, bool pdl, Args... args) {
   cudaLaunchAttribute at{};
@@ -280,6 +289,7 @@ struct SeriesPass {
   int radix[8];
 };
 constexpr int kTwFine = 2048;  // entries of the fine twiddle table
+constexpr int kPassMaxR = 1024;  // largest radix of a pass
 // passes of an N-point FFT; -1 if N has a factor other than 2, 3, 5, 7
 int series_plan(int n, SeriesPass *pass, int max_passes);
 size_t series_twiddle_count(int n);
@@ -294,6 +304,7 @@ cudaError_t launch_ftc_tc(const FtcParams &p, bool f16, cudaStream_t s);
 // factors conjugated; status / timeout as for the FT convolution
 cudaError_t launch_tile_tc(const TileParams &p, bool f16, int *status, long long timeout_ns, cudaStream_t s);
 cudaError_t launch_hsum(const HsumParams &p, const HsumMaps &m, cudaStream_t s, bool pdl = false);
+constexpr int kHsMaxSmem = 227 * 1024;  // what an SM has for one CTA
 // consumer warps of the harmonic-summing kernel for `half` (4 templates each)
 int hsum_warps(int half);
 cudaError_t launch_recheck(const RecheckParams &p, cudaStream_t s, bool pdl = false);

@@ -803,13 +803,13 @@ cudaError_t launch_ftc(const FtcParams &p, cudaStream_t s, bool pdl) {
   if ((p.variant ? p.variant : ftc_variant()) == 1 && !p.inject_stall) {  // the test hook is the pair form's
     const int smem = ex_smem_bytes();
     auto kern = p.trials ? ftc_kernel<true> : ftc_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     const long long ctas = (items + kWarpsPerCta - 1) / kWarpsPerCta;
     kern<<<(int)(ctas < n_sm ? ctas : n_sm), 256, smem, s>>>(p);
   } else if (p.ctas_per_sm != 1) {
     auto kern = p.trials ? ftcg_kernel<true> : ftcg_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
+    cudaError_t e = allow_smem(kern, kGroupSmem);
     if (e != cudaSuccess) return e;
     FtcParams q = p;
     q.group_tiles = group_tiles(p.n_tiles, p.n_rows, n_sm);
@@ -819,7 +819,7 @@ cudaError_t launch_ftc(const FtcParams &p, cudaStream_t s, bool pdl) {
   } else {
     const int smem = (kPairsPerCta * kEx2Floats + kTw2Floats) * (int)sizeof(float);
     auto kern = p.trials ? ftc2_kernel<true> : ftc2_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     const long long ctas = (items + kPairsPerCta - 1) / kPairsPerCta;
     kern<<<(int)(ctas < n_sm ? ctas : n_sm), 256, smem, s>>>(p);

@@ -1152,7 +1152,7 @@ template <int MAXP, int NW, int STAGES, int MINB>
 static cudaError_t launch_hsum_t(const HsumParams &p, const HsumMaps &m, cudaStream_t s, bool pdl) {
   const int smem = hsum_smem_bytes(p);
   auto kern = hsum_kernel<MAXP, NW, STAGES, MINB>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = allow_smem(kern, kHsMaxSmem);
   if (e != cudaSuccess) return e;
   const int n_sm = current_sm_count();
   const int items = (p.n_bins + kHsBins - 1) / kHsBins * 2;
@@ -1188,12 +1188,12 @@ cudaError_t launch_recheck(const RecheckParams &p, cudaStream_t s, bool pdl) {
 cudaError_t launch_select(const SelectParams &p, cudaStream_t s, bool pdl) {
   const int n_sm = current_sm_count();
   const int hsmem = p.n_planes * kSelBuckets * 4;
-  cudaError_t e = cudaFuncSetAttribute(select_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hsmem);
+  cudaError_t e = allow_smem(select_hist_kernel, kMaxPlanes * kSelBuckets * 4);
   if (e != cudaSuccess) return e;
   if ((e = launch_kernel(select_hist_kernel, dim3(n_sm), dim3(1024), hsmem, s, pdl, p)) != cudaSuccess) return e;
   if ((e = launch_kernel(select_gather_kernel, dim3(4 * n_sm), dim3(256), 0, s, pdl, p)) != cudaSuccess) return e;
   const int fsmem = (kSortCap + kMaxCompat) * (8 + 4);
-  e = cudaFuncSetAttribute(select_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fsmem);
+  e = allow_smem(select_finalize_kernel, fsmem);
   if (e != cudaSuccess) return e;
   return launch_kernel(select_finalize_kernel, dim3(p.n_planes, kFinSlices), dim3(1024), fsmem, s, pdl, p);
 }

@@ -379,7 +379,7 @@ cudaError_t launch_ftc_tc(const FtcParams &p, bool f16, cudaStream_t s) {
   const long long groups = ((long long)p.n_tiles * p.n_rows + kTcItems - 1) / kTcItems;
   const int grid = (int)(groups < n_sm ? groups : n_sm);
   auto kern = f16 ? ftc_tc_kernel<true, false> : ftc_tc_kernel<false, false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+  cudaError_t e = allow_smem(kern, kTcSmem);
   if (e != cudaSuccess) return e;
   kern<<<grid, kTcThreads, kTcSmem, s>>>(p);
   return cudaGetLastError();
@@ -402,7 +402,7 @@ cudaError_t launch_tile_tc(const TileParams &t, bool f16, int *status, long long
   const long long groups = ((long long)t.n_tiles + kTcItems - 1) / kTcItems;
   const int grid = (int)(groups < n_sm ? groups : n_sm);
   auto kern = f16 ? ftc_tc_kernel<true, true> : ftc_tc_kernel<false, true>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+  cudaError_t e = allow_smem(kern, kTcSmem);
   if (e != cudaSuccess) return e;
   kern<<<grid, kTcThreads, kTcSmem, s>>>(p);
   return cudaGetLastError();
