@@ -221,10 +221,7 @@ void rows_of(const fdas_handle *h, fdas_fop_part w, int *row_begin, int *n_rows)
 // ------------------------------------------------- harmonic-summing geometry
 // Box shapes of the per-item staging (see hsum_kernel): plane 1 is kHsBins bins x
 // 4 NW rows, plane j >= 2 covers bins [(f0/j) & ~3, ...) of the rows
-// trunc(|t|/j), |t| < 4 NW.  Where j divides kHsBins a block's bins f0/j .. are
-// aligned and just kHsBins / j; else up to (f0 + kHsBins - 4) / j + 1, the last
-// value the kernel reads, for any of its blocks (the shift of f0/j against its
-// 4-aligned start repeats every 4 j blocks).
+// trunc(|t|/j), |t| < 4 NW.
 void hsum_geometry(const fdas_handle *h, HsumParams &p) {
   const int nw = hsum_warps(h->H);
   p.bw[1] = kHsBins;
@@ -234,11 +231,7 @@ void hsum_geometry(const fdas_handle *h, HsumParams &p) {
   off += p.bw[1] * p.bh[1];
   unsigned bytes = (unsigned)(p.bw[1] * p.bh[1] * 4);
   for (int j = 2; j <= h->P; ++j) {
-    int width = kHsBins / j;
-    if (kHsBins % j)
-      for (int f0 = 0; f0 < 4 * j * kHsBins; f0 += kHsBins)
-        width = std::max(width, (f0 + kHsBins - 4) / j + 2 - ((f0 / j) & ~3));
-    p.bw[j] = (width + 3) & ~3;
+    p.bw[j] = hs_box_width(j);
     p.bh[j] = (4 * nw - 1) / j + 1;
     off = (off + 31) & ~31;  // 128-byte aligned TMA destinations
     p.soff[j] = off;

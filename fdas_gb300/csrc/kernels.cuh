@@ -5,11 +5,12 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "hsum_boxes.cuh"
+
 namespace fdas {
 
 constexpr int kTile = 2048;          // FFT / tile size (gen_info.h:33, 42)
 constexpr int kMaxPlanes = 16;       // harmonic planes supported by the kernels
-constexpr int kHsBins = 256;         // bins per harmonic-summing work item
 constexpr int kSortCap = 8192;       // boundary records one CTA ranks in shared memory
 constexpr int kMaxCompat = 2048;     // entries per plane of the fixed-size list
 constexpr int kSelBuckets = 2048;    // power buckets of the top-K selection (float bits 30..20)

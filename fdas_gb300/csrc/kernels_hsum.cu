@@ -79,8 +79,8 @@ struct EmitBuf {
 // hardware (they only feed masked cells).  kHsStages stages deep: full / empty
 // mbarriers, every wait bounded by %globaltimer.
 //
-// Planes 2, 4 and 8 read their values with 8- and 4-byte loads at
-// compile-time offsets; for planes 3, 5, 6, 7 the eight bins map onto offsets
+// Planes 2, 4, 8 and 16 read their values with 8- and 4-byte loads at
+// compile-time offsets; for the others the eight bins map onto offsets
 // from two divisions per plane and the four rows onto two staged rows split at
 // a warp-uniform point, handled by a switch.
 //
@@ -362,7 +362,7 @@ __device__ __forceinline__ unsigned hs_exact_marks(const HsumParams &p, const fl
       const int a0 = (f0 / j) & ~3;
       const int bw = p.bw[j], bh = p.bh[j];
       const float *box = stage + p.soff[j];
-      // f0 is a multiple of 256, so for j = 2, 4, 8 the box starts at f0 / j
+      // f0 is a multiple of 256, so for j = 2, 4, 8, 16 the box starts at f0 / j
       float vmax;
       if constexpr (j == 2) {
         const float *r0 = box + srow(t0 / 2, bh, sgn) * bw + 2 * lane;
@@ -378,17 +378,9 @@ __device__ __forceinline__ unsigned hs_exact_marks(const HsumParams &p, const fl
           add2(acc[kk][4], acc[kk][5], vb.x, vb.x);
           add2(acc[kk][6], acc[kk][7], vb.y, vb.y);
         }
-      } else if constexpr (j == 4) {
-        const float *r0 = box + srow(t0 / 4, bh, sgn) * bw + lane;
-        const float va = r0[0], vb = r0[32];
-        vmax = fmaxf(va, vb);
-  #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-  #pragma unroll
-          for (int e = 0; e < 8; e += 2) add2(acc[kk][e], acc[kk][e + 1], e < 4 ? va : vb, e < 4 ? va : vb);
-      } else if constexpr (j == 8) {
-        const float *r0 = box + srow(t0 / 8, bh, sgn) * bw + (lane >> 1);
-        const float va = r0[0], vb = r0[16];
+      } else if constexpr (hs_one_value(j)) {  // planes 4, 8 and 16: one value per group
+        const float *r0 = box + srow(t0 / j, bh, sgn) * bw + lane / (j / 4);
+        const float va = r0[0], vb = r0[128 / j];
         vmax = fmaxf(va, vb);
   #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
@@ -489,7 +481,7 @@ __device__ __forceinline__ void hs_bound_plane(HsBounds &u, const float *stage, 
     const float2 a0 = q0[0], b0 = q0[32], a1 = q1[0], b1 = q1[32];
     u.a += fmaxf(fmax3(a0.x, a0.y, a1.x), a1.y);
     u.b += fmaxf(fmax3(b0.x, b0.y, b1.x), b1.y);
-  } else if constexpr (j == 4 || j == 8 || j == 16) {  // one value for the group
+  } else if constexpr (hs_one_value(j)) {  // one value for the group
     const float *q = stage + r0 + lane / (j / 4);
     u.a += q[0];
     u.b += q[128 / j];
