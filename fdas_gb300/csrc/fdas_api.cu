@@ -327,14 +327,18 @@ unsigned long long *stamp_at(const BufferSet &S, int i) {
 // a capture).  The tiling then zeroes the control words for all of them, and
 // kernels may start on the tail of the one before (programmatic dependent launch).
 // Not where a later stage would be refused, whose call leaves the earlier
-// search's counts alone, nor for the tensor-core tiling, which zeroes nothing.
+// search's counts alone, nor for the tensor-core tiling, which zeroes nothing, nor
+// under sync_pipeline, whose other set waits for the event after the FT convolution
+// (and whose harmonic summing, held back, leaves the earlier search's results until
+// it runs).
 bool can_chain(const fdas_handle *h, int ab, const float *thr) {
   const BufferSet &S = h->set[ab];
+  if (h->cfg.precision || h->cfg.sync_pipeline || !S.have_templates || (!thr && S.thresholds.empty())) return false;
   HsumParams p{};
   p.half = h->H;
   p.n_planes = h->P;
   hsum_geometry(h, p);
-  return !h->cfg.precision && S.have_templates && (thr || !S.thresholds.empty()) && hsum_smem_bytes(p) <= kHsMaxSmem;
+  return hsum_smem_bytes(p) <= kHsMaxSmem;
 }
 
 fdas_status enqueue_tiling(fdas_handle *h, int ab, bool chain) {
@@ -411,8 +415,8 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which, bool chain)
   if (chain) p.stamp = stamp_at(S, 1);
   CK(h, launch_ftc(p, S.stream, chain));
   if (!chain) CK(h, cudaEventRecord(S.ev[3], S.stream));
+  S.ev_ftc_recorded = !chain;
   S.ftc_unchecked = true;
-  S.ev_ftc_recorded = true;
   S.fop_from_input = true;
   return FDAS_OK;
 }
@@ -1163,8 +1167,7 @@ fdas_status fdas_launch(fdas_handle *h, const fdas_complex *input, const float *
   if (h->cfg.sync_pipeline && (st = release_pending(h, 1 - ab)) != FDAS_OK) return st;
   long long t[5];  // steady-clock times around the enqueue steps (FDAS.cpp:556-566)
   t[0] = steady_ns();
-  // (a held-back harmonic summing keeps the earlier search's results until it runs)
-  const bool chain = !h->cfg.sync_pipeline && can_chain(h, ab, thresholds);
+  const bool chain = can_chain(h, ab, thresholds);
   if ((st = enqueue_input(h, ab, input, false, chain)) != FDAS_OK) return st;
   if ((st = enqueue_tiling(h, ab, chain)) != FDAS_OK) return st;
   t[1] = steady_ns();

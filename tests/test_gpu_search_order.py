@@ -1,0 +1,53 @@
+"""Order between the two buffer sets' searches, read from their event times."""
+import io
+
+import numpy as np
+import pytest
+
+from gpu_util import make_pipeline
+from fdas_gb300.fdas import FDAS
+from fdas_gb300.templates import template_bank
+from oracle import fdas_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+N = 1 << 20  # an FT convolution of about 150 us, several times the time to enqueue a search
+FIELDS = ("in_begin", "in_end", "tile_begin", "tile_end", "ftc_begin", "ftc_end", "hsum_begin", "hsum_end",
+          "list_begin", "list_end")
+
+
+def noise(seed):
+    rng = np.random.default_rng(seed)
+    return ((rng.standard_normal(N) + 1j * rng.standard_normal(N)) * np.sqrt(0.5)).astype(np.complex64)
+
+
+def handle(log, **kw):
+    p = make_pipeline(N, log=log, **kw)
+    for ab in (FDAS.A, FDAS.B):
+        assert p.upload_templates(template_bank(), ab)
+    return p
+
+
+def events(p, log, ab):
+    at = len(log.getvalue())
+    p.print_events(ab)
+    line = [s for s in log.getvalue()[at:].splitlines() if s.startswith("@@@")][-1]
+    return dict(zip(FIELDS, (int(v) for v in line.split(",")[2:])))
+
+
+@pytest.mark.parametrize("order", [(FDAS.A, FDAS.B), (FDAS.B, FDAS.A)])
+def test_device_searches_under_sync_pipeline(order):
+    """sync_pipeline: the tiling of one set waits for the other's FT convolution, for
+    searches of device spectra as for launches."""
+    import torch
+    log, thr = io.StringIO(), O.chi2_thresholds(1e-7, 8)
+    p = handle(log, sync_pipeline=True)
+    x = torch.from_numpy(noise(1).view(np.float32)).cuda()
+    torch.cuda.synchronize()
+    for rep in range(3):
+        for ab in order:
+            assert p.enqueue_search_device(x.data_ptr(), thr, FDAS.AllAccelerations, ab), p.last_error
+        for ab in order:
+            assert p.synchronize(ab)
+    first, second = (events(p, log, ab) for ab in order)
+    assert second["tile_begin"] >= first["ftc_end"] - 1000  # (ns; the times are floats in ms)
