@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #include "hsum_boxes.cuh"
 
 namespace fdas {
@@ -51,15 +53,6 @@ __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.la
 __device__ __forceinline__ void stamp(unsigned long long *at) {
   if (at && blockIdx.x == 0 && threadIdx.x == 0) asm volatile("mov.u64 %0, %globaltimer;" : "=l"(*at));
 }
-// Lets a kernel be launched with up to `bytes` of dynamic shared memory.  The limit is
-// one per kernel and device, shared by every handle and thread: `bytes` is the most that
-// any launch of the kernel takes, never this launch's own, or a thread with a smaller
-// launch would lower it between another's call and its launch (which then fails: 18 of
-// 2000 series FFTs of 2^20 points beside a thread with 4096).
-template <typename Kernel>
-cudaError_t allow_smem(Kernel kern, int bytes) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
 template <typename Kernel, typename... Args>
 cudaError_t launch_kernel(Kernel kern, dim3 grid, dim3 block, int smem, cudaStream_t s, bool pdl, Args... args) {
   cudaLaunchAttribute at{};
@@ -73,6 +66,28 @@ cudaError_t launch_kernel(Kernel kern, dim3 grid, dim3 block, int smem, cudaStre
   c.attrs = &at;
   c.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&c, kern, args...);
+}
+// Lets a kernel be launched with `bytes` of dynamic shared memory, every launch of it alike.
+template <typename Kernel>
+cudaError_t allow_smem(Kernel kern, int bytes) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+// A kernel whose launches differ in shared memory.  The limit is one per kernel and
+// device, shared by every handle and thread, so setting it and launching are one step
+// under a lock: else a thread with a smaller launch lowers it between another's call and
+// its launch, which then fails (18 of 2000 series FFTs of 2^20 points beside a thread
+// with 4096).  One limit for all of a kernel's launches instead makes searches that run
+// side by side slower (eight served requests 770 -> 800 us with harmonic summing and
+// the histogram at their largest): what an SM sets aside follows the limit, not the launch.
+inline std::mutex &smem_limit_lock() {
+  static std::mutex lock;
+  return lock;
+}
+template <typename Kernel, typename... Args>
+cudaError_t launch_sized(Kernel kern, dim3 grid, dim3 block, int smem, cudaStream_t s, bool pdl, Args... args) {
+  const std::lock_guard<std::mutex> hold(smem_limit_lock());
+  const cudaError_t e = allow_smem(kern, smem);
+  return e != cudaSuccess ? e : launch_kernel(kern, grid, block, smem, s, pdl, args...);
 }
 
 // ---- (a) overlap-save tiling + forward FFT (tile_input.cl.mako, fft_4p.cl)
@@ -290,7 +305,6 @@ struct SeriesPass {
   int radix[8];
 };
 constexpr int kTwFine = 2048;  // entries of the fine twiddle table
-constexpr int kPassMaxR = 1024;  // largest radix of a pass
 // passes of an N-point FFT; -1 if N has a factor other than 2, 3, 5, 7
 int series_plan(int n, SeriesPass *pass, int max_passes);
 size_t series_twiddle_count(int n);

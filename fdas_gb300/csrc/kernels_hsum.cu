@@ -1144,11 +1144,9 @@ template <int MAXP, int NW, int STAGES, int MINB>
 static cudaError_t launch_hsum_t(const HsumParams &p, const HsumMaps &m, cudaStream_t s, bool pdl) {
   const int smem = hsum_smem_bytes(p);
   auto kern = hsum_kernel<MAXP, NW, STAGES, MINB>;
-  cudaError_t e = allow_smem(kern, kHsMaxSmem);
-  if (e != cudaSuccess) return e;
   const int n_sm = current_sm_count();
   const int items = (p.n_bins + kHsBins - 1) / kHsBins * 2;
-  return launch_kernel(kern, dim3(items < n_sm ? items : n_sm), dim3(32 * (NW + 1)), smem, s, pdl, p, m);
+  return launch_sized(kern, dim3(items < n_sm ? items : n_sm), dim3(32 * (NW + 1)), smem, s, pdl, p, m);
 }
 
 cudaError_t launch_hsum(const HsumParams &p, const HsumMaps &m, cudaStream_t s, bool pdl) {
@@ -1180,9 +1178,8 @@ cudaError_t launch_recheck(const RecheckParams &p, cudaStream_t s, bool pdl) {
 cudaError_t launch_select(const SelectParams &p, cudaStream_t s, bool pdl) {
   const int n_sm = current_sm_count();
   const int hsmem = p.n_planes * kSelBuckets * 4;
-  cudaError_t e = allow_smem(select_hist_kernel, kMaxPlanes * kSelBuckets * 4);
+  cudaError_t e = launch_sized(select_hist_kernel, dim3(n_sm), dim3(1024), hsmem, s, pdl, p);
   if (e != cudaSuccess) return e;
-  if ((e = launch_kernel(select_hist_kernel, dim3(n_sm), dim3(1024), hsmem, s, pdl, p)) != cudaSuccess) return e;
   if ((e = launch_kernel(select_gather_kernel, dim3(4 * n_sm), dim3(256), 0, s, pdl, p)) != cudaSuccess) return e;
   const int fsmem = (kSortCap + kMaxCompat) * (8 + 4);
   e = allow_smem(select_finalize_kernel, fsmem);

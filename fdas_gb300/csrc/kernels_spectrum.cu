@@ -341,7 +341,7 @@ int series_plan(int n, SeriesPass *pass, int max_passes) {
   // two passes of up to 1024 instead of three of about 100 from 655360 points on, where
   // a pass more costs more than its CTAs of 8192 points wait (device samples, two
   // against three: 524288 34.5 / 31.5 us, 700000 35 / 35, 800000 36.0 / 39.8, 2^20 38 / 40.5, 10^6 37 / 42.5)
-  if (n > 655360 && n <= 1024 * 1024) count = 2, max_r = kPassMaxR;
+  if (n > 655360 && n <= 1024 * 1024) count = 2, max_r = 1024;
   for (;; ++count) {
     if (count > max_passes) return -1;
     int R[16];
@@ -383,9 +383,6 @@ cudaError_t launch_series_twiddles(float4 *tw, int n, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Twiddles and two buffers of the largest radix in 8 columns (more columns only while
-// a buffer's points stay within 2048)
-constexpr int kPassMaxSmem = (2 * kPassMaxR + 2 * kPassMaxR * (8 + 1)) * (int)sizeof(float2);
 cudaError_t launch_series_spectrum(const SeriesParams &p, cudaStream_t s) {
   SeriesPass pass[16];
   const int np = series_plan(p.n, pass, 16);
@@ -400,10 +397,8 @@ cudaError_t launch_series_spectrum(const SeriesParams &p, cudaStream_t s) {
     const SeriesPass &q = pass[i];
     const int buffers = std::min(q.n_steps - 1, 2);
     const int smem = (2 * q.R + buffers * q.R * (q.B + 1)) * (int)sizeof(float2);
-    cudaError_t e = allow_smem(series_pass_kernel, kPassMaxSmem);
-    if (e != cudaSuccess) return e;
-    e = launch_kernel(series_pass_kernel, (unsigned)((q.m + q.B - 1) / q.B), q.threads, smem, s, chained, cur, dst,
-                      q, p.tw);
+    const cudaError_t e = launch_sized(series_pass_kernel, (unsigned)((q.m + q.B - 1) / q.B), q.threads, smem, s,
+                                       chained, cur, dst, q, p.tw);
     if (e != cudaSuccess) return e;
     chained = true;
     cur = dst;
