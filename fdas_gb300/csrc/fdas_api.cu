@@ -41,8 +41,10 @@ constexpr int kCtrlBound = kCtrlItems + 1;           // + plane: boundary record
 constexpr int kCtrlWords = kCtrlBound + kMaxPlanes;   // zeroed before every harmonic summing
 constexpr int kCtrlFtcStatus = kCtrlWords;           // FT-convolution status, zeroed before each FT convolution
 constexpr int kCtrlTileStatus = kCtrlWords + 1;      // tiling status (tensor-core form), zeroed before each tiling
-constexpr int kCtrlZeroed = kCtrlWords + 2;           // words a search starts from zero
-constexpr int kCtrlStamp = (kCtrlZeroed + 1) & ~1;   // three 64-bit times: start of tiling, FT convolution, harmonic summing
+// three 64-bit times: end of FT convolution (the latest CTA's), tiling, search
+constexpr int kCtrlStamp = (kCtrlWords + 3) & ~1;
+constexpr int kCtrlZeroed = kCtrlStamp + 2;          // words a search starts from zero
+constexpr int kEndFtc = 0, kEndTiling = 1, kEndSearch = 2;
 constexpr int kCtrlStride = kCtrlStamp + 6;          // control words per buffer set
 constexpr uint32_t kDefaultCapacity = 1u << 22;     // candidate records per buffer set
 constexpr uint32_t kMaxCapacity = 1u << 27;
@@ -366,12 +368,12 @@ fdas_status enqueue_tiling(fdas_handle *h, int ab, bool chain) {
     if (chain) {
       p.zero = S.d_ctrl;
       p.n_zero = kCtrlZeroed;
-      p.stamp = stamp_at(S, 0);
+      p.stamp = stamp_at(S, kEndTiling);
     }
     CK(h, launch_tile_fft(p, S.stream));
   }
   // an event between two kernels keeps the second from starting early (about 2 us
-  // each): in a chain the kernels write down their start times instead
+  // each): in a chain the kernels write down their end times instead
   S.stamped = chain;
   if (!chain) CK(h, cudaEventRecord(S.ev[2], S.stream));
   return FDAS_OK;
@@ -412,7 +414,7 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which, bool chain)
   if (S.input_from_host && !h->cfg.overlap && !h->cfg.sync_pipeline && h->set[1 - ab].ev_hsum_recorded)
     CK(h, cudaStreamWaitEvent(S.stream, h->set[1 - ab].ev_hsum, 0));
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl + kCtrlFtcStatus, 0, sizeof(unsigned), S.stream));
-  if (chain) p.stamp = stamp_at(S, 1);
+  if (chain) p.stamp = stamp_at(S, kEndFtc);
   CK(h, launch_ftc(p, S.stream, chain));
   if (!chain) CK(h, cudaEventRecord(S.ev[3], S.stream));
   S.ev_ftc_recorded = !chain;
@@ -475,7 +477,6 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
     return fail(h, FDAS_ERR_UNSUPPORTED, "harmonic summing staging exceeds shared memory (too many templates x planes)");
   S.ctrl_valid = S.results_on_host = false;  // until the kernels that write them are enqueued
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl, 0, sizeof(unsigned) * kCtrlWords, S.stream));
-  if (chain) p.stamp = stamp_at(S, 2);
   CK(h, launch_hsum(p, S.maps, S.stream, chain));
   // (the batched form's per-trial views have none; with one set in use nobody waits for it)
   if (S.ev_hsum && (!chain || h->set[1 - ab].used)) {
@@ -524,7 +525,8 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   f.status = p.status;
   f.ctrl = S.d_ctrl;
   f.host_ctrl = S.h_ctrl;
-  f.n_ctrl = kCtrlStride;
+  f.n_ctrl = kCtrlStamp + 4;
+  f.stamp = chain ? reinterpret_cast<unsigned long long *>(S.h_ctrl + kCtrlStamp) + kEndSearch : nullptr;
   // Host memory written by the kernels saves each retrieval its copies (four from
   // pageable memory: 55 us for 442 records before, 20 after)
   f.host_loc = S.h_cloc;
@@ -646,7 +648,10 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
-// ms of tiling, FT convolution and harmonic summing of a completed search
+// ms of tiling, FT convolution and harmonic summing of a completed search: each from
+// the end of the one before, so that a wait (for the other set's kernels) counts
+// for the stage that waited.  In a chain the tiling gets what the events around it
+// leave beside the kernels' end times.
 void stage_times(const BufferSet &S, float *ms3) {
   if (!S.stamped) {
     const int at[4] = {S.ev_in, 2, 3, S.ev_hs};
@@ -655,9 +660,9 @@ void stage_times(const BufferSet &S, float *ms3) {
   }
   unsigned long long t[3];
   std::memcpy(t, S.h_ctrl + kCtrlStamp, sizeof(t));
-  ms3[0] = (float)(1e-6 * (double)(long long)(t[1] - t[0]));
-  ms3[1] = (float)(1e-6 * (double)(long long)(t[2] - t[1]));
-  ms3[2] = std::max(0.f, elapsed(S.ev[S.ev_in], S.ev[S.ev_hs]) - ms3[0] - ms3[1]);
+  ms3[1] = std::max(0.f, (float)(1e-6 * (double)(long long)(t[kEndFtc] - t[kEndTiling])));
+  ms3[2] = std::max(0.f, (float)(1e-6 * (double)(long long)(t[kEndSearch] - t[kEndFtc])));
+  ms3[0] = std::max(0.f, elapsed(S.ev[S.ev_in], S.ev[S.ev_hs]) - ms3[1] - ms3[2]);
 }
 
 // Layout of a set's host memory from `base` (host_bytes() bytes, 16-byte aligned)
@@ -1487,8 +1492,8 @@ void fdas_print_events(fdas_handle *h, fdas_buffer_set ab) {
   if (S.stamped) {
     float st[3];
     stage_times(S, st);
-    t[2] = std::min(t[4], t[1] + (long long)llround(1e6 * (double)st[0]));
-    t[3] = std::min(t[4], t[2] + (long long)llround(1e6 * (double)st[1]));
+    t[3] = std::max(t[1], t[4] - (long long)llround(1e6 * (double)st[2]));
+    t[2] = std::max(t[1], t[3] - (long long)llround(1e6 * (double)st[1]));
   }
   logf(h, "@@@,%c,%lld,%lld,%lld,%lld,%lld,%lld,%lld,%lld,%lld,%lld", ab == FDAS_SET_A ? 'A' : 'B', t[0], t[1], t[1],
        t[2], t[2], t[3], t[3], t[4], t[4], t[5]);

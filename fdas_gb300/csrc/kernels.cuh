@@ -48,10 +48,19 @@ __host__ __device__ inline unsigned long long cand_key(int plane, int row, int b
 // between its kernels and copies after them, of 2^21 bins 699 -> 691 -> 678.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// %globaltimer (32 ns steps here) written by one thread of a kernel where its
-// part of the search starts, or nothing
-__device__ __forceinline__ void stamp(unsigned long long *at) {
-  if (at && blockIdx.x == 0 && threadIdx.x == 0) asm volatile("mov.u64 %0, %globaltimer;" : "=l"(*at));
+// Where a kernel's work ends, by %globaltimer (32 ns steps here), or nothing: written by
+// its last block (blocks start in order, so short ones of equal work end within a
+// block's time of it), or the latest of all blocks, into a word that starts from zero.
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ void stamp_last_block(unsigned long long *at) {
+  if (at && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && threadIdx.x == 0) *at = global_ns();
+}
+__device__ __forceinline__ void stamp_latest(unsigned long long *at) {
+  if (at && threadIdx.x == 0) atomicMax(at, global_ns());
 }
 template <typename Kernel, typename... Args>
 cudaError_t launch_kernel(Kernel kern, dim3 grid, dim3 block, int smem, cudaStream_t s, bool pdl, Args... args) {
@@ -133,7 +142,7 @@ struct TileParams {
   int tmpl_p4 = 0;           // the source is in p4 order
   unsigned *zero = nullptr;  // words to zero before the following kernels run (a search's control words)
   int n_zero = 0;
-  unsigned long long *stamp = nullptr;  // start time (stage times of a search enqueued in one go)
+  unsigned long long *stamp = nullptr;  // end time (stage times of a search enqueued in one go)
 };
 
 // ---- (c) template multiply + inverse FFT + |.|^2 + discard (mux_and_mult,
@@ -203,7 +212,6 @@ struct HsumParams {
   int lean;               // 1: fewer stages and registers (shares an SM with the FT convolution)
   int inject_stall = 0;   // test hook: the first stage of every CTA is announced on its barriers
                           // but its copies are not issued, so the consumers' waits run out
-  unsigned long long *stamp = nullptr;
 };
 
 // 2-D tensor maps of the FOP (rows x stride floats), one box shape per plane
@@ -263,6 +271,7 @@ struct SelectParams {
   const unsigned *ctrl;   // n_ctrl control words, copied to pinned host memory at the end
   unsigned *host_ctrl;
   int n_ctrl;
+  unsigned long long *stamp;  // end time, in pinned host memory
 };
 
 // ---- template spectra / taps in FP64

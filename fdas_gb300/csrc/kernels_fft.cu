@@ -74,10 +74,8 @@ __global__ void __launch_bounds__(kTileThreads, 8) tile_fft_kernel(TileParams p)
     local = tile - tr.tile_begin;
   }
   grid_wait();
-  if (blockIdx.x == 0 && p.n_zero) {
-    stamp(p.stamp);
+  if (blockIdx.x == 0)
     for (int i = t; i < p.n_zero; i += kTileThreads) p.zero[i] = 0u;
-  }
   const long long start = local * p.payload - p.overlap + t;
   float2 v[16];
   sfor<16>([&](auto N1) {
@@ -134,6 +132,7 @@ __global__ void __launch_bounds__(kTileThreads, 8) tile_fft_kernel(TileParams p)
       out[128 * c + 256 * k] = u[k];
     });
   });
+  stamp_last_block(p.stamp);
 }
 
 // ------------------------------------------------------------ TMA helpers
@@ -248,7 +247,6 @@ __global__ void __launch_bounds__(256, 1) ftc_kernel(FtcParams p) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
-  stamp(p.stamp);
   const TwiddleBases tb = load_twiddle_bases<+1>(p.twiddle, lane);
   if (item < n_items && lane == 0)
     prefetch_template(ex, p.tmpl + (long long)(p.row_begin + item % p.n_rows) * kTile, bar);
@@ -293,6 +291,7 @@ __global__ void __launch_bounds__(256, 1) ftc_kernel(FtcParams p) {
       });
     });
   }
+  stamp_latest(p.stamp);
 }
 
 // ---------------------------------------------------------------------------
@@ -340,7 +339,6 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   fill_twiddle2(twt, p.twiddle);
-  stamp(p.stamp);
   __syncthreads();
   if (item < n_items && tp == 0) {
     if (p.inject_stall) mbar_arrive_expect_tx(bar, kTile * 8);  // test hook: a copy that never comes
@@ -411,6 +409,7 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
     tile = next_tile;
     rr = next_rr;
   }
+  stamp_latest(p.stamp);
 }
 
 // ---------------------------------------------------------------------------
@@ -564,7 +563,6 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     grid_wait();
-    stamp(p.stamp);
     if (threadIdx.x == 0)
       for (int i = 0; i < kGroupRing && i < steps; ++i) {
         if (i == 0 && p.inject_stall) {  // test hook: a copy that never comes
@@ -695,6 +693,7 @@ __global__ void __launch_bounds__(64 * kGroupPairs, 1) ftcg_kernel(FtcParams p) 
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  stamp_latest(p.stamp);
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(ring.tmem), "r"(kGroupTmemCols));

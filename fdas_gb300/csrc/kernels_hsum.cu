@@ -632,7 +632,6 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
   }
   grid_release();
   grid_wait();
-  stamp(p.stamp);
   __syncthreads();
 
   if (warp == NW) {
@@ -1120,6 +1119,7 @@ __global__ void __launch_bounds__(1024) select_finalize_kernel(SelectParams p) {
   for (int i = max(lo, kept) + (int)threadIdx.x; i < hi; i += blockDim.x) {
     put(i, p.invalid_location, -1.0f);
   }
+  stamp_last_block(p.stamp);
 }
 
 // ----------------------------------------------------------------- launchers

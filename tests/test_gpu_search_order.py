@@ -51,3 +51,41 @@ def test_device_searches_under_sync_pipeline(order):
             assert p.synchronize(ab)
     first, second = (events(p, log, ab) for ab in order)
     assert second["tile_begin"] >= first["ftc_end"] - 1000  # (ns; the times are floats in ms)
+
+
+def launched(p, xs, outs, thr, order):
+    for x, (loc, pwr), ab in zip(xs, outs, order):
+        assert p.launch(x.array, thr, loc.array, pwr.array, FDAS.AllAccelerations, ab), p.last_error
+    for ab in order:
+        assert p.wait(ab)
+
+
+def host_arrays(p, count):
+    from fdas_gb300.fdas import PinnedArray
+    nc = p.get_candidate_list_sz()
+    xs = [PinnedArray((N,), np.complex64) for _ in range(count)]
+    for i, x in enumerate(xs):
+        x.array[:] = noise(i)
+    return xs, [(PinnedArray((nc,), np.uint32), PinnedArray((nc,), np.float32)) for _ in range(count)]
+
+
+def test_stage_times_of_a_search_that_waits():
+    """The second of two launches waits for the first: its harmonic summing, which runs
+    by itself, takes as long as a lone search's, and its stages fill its total."""
+    log, thr = io.StringIO(), O.chi2_thresholds(1e-7, 8)
+    p = handle(log)
+    xs, outs = host_arrays(p, 2)
+    for _ in range(2):
+        launched(p, xs, outs, thr, (FDAS.A, FDAS.B))
+    launched(p, xs[1:], outs[1:], thr, (FDAS.B,))
+    lone = p.stage_times(FDAS.B)
+    launched(p, xs, outs, thr, (FDAS.A, FDAS.B))
+    both = p.stage_times(FDAS.B)
+    print(lone, p.stage_times(FDAS.A), both)
+    assert lone[1] < 0.5 * lone[2] and lone[3] > 0  # (tiling is a tenth of the FT convolution)
+    assert both[2] > 0.9 * lone[2]
+    assert both[3] < 1.25 * lone[3] + 0.01
+    assert abs(both[:5].sum() - both[5]) < 0.005
+    at = events(p, log, FDAS.B)
+    assert list(at.values()) == sorted(at.values())
+    assert abs(1e-6 * (at["hsum_end"] - at["hsum_begin"]) - both[3]) < 0.001
