@@ -101,6 +101,7 @@ struct BufferSet {
   bool tile_unchecked = false; // a tensor-core tiling ran whose status word has not been checked
   cudaEvent_t ev_hsum = nullptr;  // end of this set's last harmonic-summing kernel
   bool ev_hsum_recorded = false;
+  bool hsum_unmarked = false;     // the last harmonic summing has no such event yet
   bool input_from_host = false;   // the current spectrum was copied in from host memory
   const float2 *host_input = nullptr;  // read by the next tiling instead of d_input, which it fills
   // events that end the input copy and the harmonic summing: the launch's first and
@@ -411,8 +412,15 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which, bool chain)
   // 16 MB copy and tiling -- starts on an empty GPU every second search.
   // Device-resident searches queued ahead keep the unordered form, where the
   // two harmonic summings run side by side after both FT convolutions.
-  if (S.input_from_host && !h->cfg.overlap && !h->cfg.sync_pipeline && h->set[1 - ab].ev_hsum_recorded)
-    CK(h, cudaStreamWaitEvent(S.stream, h->set[1 - ab].ev_hsum, 0));
+  if (S.input_from_host && !h->cfg.overlap && !h->cfg.sync_pipeline) {
+    BufferSet &other = h->set[1 - ab];
+    if (other.hsum_unmarked) {  // enqueued before this set was in use: the end of that whole search
+      CK(h, cudaEventRecord(other.ev_hsum, other.stream));
+      other.ev_hsum_recorded = true;
+      other.hsum_unmarked = false;
+    }
+    if (other.ev_hsum_recorded) CK(h, cudaStreamWaitEvent(S.stream, other.ev_hsum, 0));
+  }
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl + kCtrlFtcStatus, 0, sizeof(unsigned), S.stream));
   if (chain) p.stamp = stamp_at(S, kEndFtc);
   CK(h, launch_ftc(p, S.stream, chain));
@@ -478,10 +486,14 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   S.ctrl_valid = S.results_on_host = false;  // until the kernels that write them are enqueued
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl, 0, sizeof(unsigned) * kCtrlWords, S.stream));
   CK(h, launch_hsum(p, S.maps, S.stream, chain));
-  // (the batched form's per-trial views have none; with one set in use nobody waits for it)
-  if (S.ev_hsum && (!chain || h->set[1 - ab].used)) {
-    CK(h, cudaEventRecord(S.ev_hsum, S.stream));
-    S.ev_hsum_recorded = true;
+  // (the batched form's per-trial views have none; with one set in use it is left to the
+  // first launch on the other set, which waits for it)
+  if (S.ev_hsum) {
+    S.hsum_unmarked = chain && !h->set[1 - ab].used;
+    if (!S.hsum_unmarked) {
+      CK(h, cudaEventRecord(S.ev_hsum, S.stream));
+      S.ev_hsum_recorded = true;
+    }
   }
   if (recheck) {
     RecheckParams r{};

@@ -89,3 +89,19 @@ def test_stage_times_of_a_search_that_waits():
     at = events(p, log, FDAS.B)
     assert list(at.values()) == sorted(at.values())
     assert abs(1e-6 * (at["hsum_end"] - at["hsum_begin"]) - both[3]) < 0.001
+
+
+@pytest.mark.parametrize("order", [(FDAS.A, FDAS.B), (FDAS.B, FDAS.A)])
+def test_first_launch_on_the_second_set(order):
+    """The FT convolution of a host spectrum waits for the other set's harmonic summing
+    from the first launch on the second set on: it ends a whole FT convolution later."""
+    log, thr = io.StringIO(), O.chi2_thresholds(1e-7, 8)
+    for _ in range(2):  # (the first handle loads the kernels)
+        p = handle(log)
+        xs, outs = host_arrays(p, 2)
+        launched(p, xs[:1], outs[:1], thr, order[:1])
+        lone = events(p, log, order[0])
+        launched(p, xs, outs, thr, order)
+        first, second = (events(p, log, ab) for ab in order)
+        p.close()
+    assert second["ftc_end"] - first["hsum_end"] >= 0.8 * (lone["ftc_end"] - lone["ftc_begin"])
