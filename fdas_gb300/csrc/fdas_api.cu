@@ -326,6 +326,11 @@ unsigned long long *stamp_at(const BufferSet &S, int i) {
   return reinterpret_cast<unsigned long long *>(S.d_ctrl + kCtrlStamp) + i;
 }
 
+bool capturing(const BufferSet &S) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(S.stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
 // `chain`: the stages of one search are enqueued in one go (not a stage call, not
 // a capture).  The tiling then zeroes the control words for all of them, and
 // kernels may start on the tail of the one before (programmatic dependent launch).
@@ -333,10 +338,11 @@ unsigned long long *stamp_at(const BufferSet &S, int i) {
 // search's counts alone, nor for the tensor-core tiling, which zeroes nothing, nor
 // under sync_pipeline, whose other set waits for the event after the FT convolution
 // (and whose harmonic summing, held back, leaves the earlier search's results until
-// it runs).
+// it runs), nor where the set's stream is being captured.
 bool can_chain(const fdas_handle *h, int ab, const float *thr) {
   const BufferSet &S = h->set[ab];
-  if (h->cfg.precision || h->cfg.sync_pipeline || !S.have_templates || (!thr && S.thresholds.empty())) return false;
+  if (h->cfg.precision || h->cfg.sync_pipeline || !S.have_templates || (!thr && S.thresholds.empty()) || capturing(S))
+    return false;
   HsumParams p{};
   p.half = h->H;
   p.n_planes = h->P;
@@ -487,10 +493,13 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl, 0, sizeof(unsigned) * kCtrlWords, S.stream));
   CK(h, launch_hsum(p, S.maps, S.stream, chain));
   // (the batched form's per-trial views have none; with one set in use it is left to the
-  // first launch on the other set, which waits for it)
+  // first launch on the other set, which waits for it; in a capture the event would be
+  // the graph's, and no stream outside could wait for it)
   if (S.ev_hsum) {
+    const bool captured = !chain && capturing(S);
     S.hsum_unmarked = chain && !h->set[1 - ab].used;
-    if (!S.hsum_unmarked) {
+    if (captured) S.ev_hsum_recorded = false;
+    else if (!S.hsum_unmarked) {
       CK(h, cudaEventRecord(S.ev_hsum, S.stream));
       S.ev_hsum_recorded = true;
     }
