@@ -1149,10 +1149,11 @@ fdas_status fdas_series_to_spectrum(fdas_handle *h, const float *samples, uint64
   if (h->series_tw_n != h->N) {
     if (!h->d_series_tw)  // (a reshape only makes N smaller)
       CK(h, cudaMalloc(&h->d_series_tw, sizeof(float4) * series_twiddle_count(h->alloc_N)));
+    // (nothing reads another N's table now: this call waits for its stream before it
+    // returns, and a reshape, which alone changes N, for both; the table counts as made
+    // once it is, for the other set's stream too)
     h->series_tw_n = 0;
-    CK(h, cudaDeviceSynchronize());  // the other set may still read the table
     CK(h, launch_series_twiddles(h->d_series_tw, h->N, S.stream));
-    h->series_tw_n = h->N;
   }
   // device samples are read where they are (as pairs, so 8-byte aligned ones)
   const size_t sample_bytes = sizeof(float) * 2 * (size_t)h->N;
@@ -1173,6 +1174,7 @@ fdas_status fdas_series_to_spectrum(fdas_handle *h, const float *samples, uint64
   if (spectrum && !p.host)
     CK(h, cudaMemcpyAsync(spectrum, S.d_input, sizeof(float2) * (size_t)h->N, cudaMemcpyDeviceToHost, S.stream));
   CK(h, cudaStreamSynchronize(S.stream));
+  h->series_tw_n = h->N;
   S.series_spectrum = true;
   S.have_input = false;  // the tiles buffer was used as scratch
   logf(h, "[INFO] Spectrum of %llu samples -> %d bins", (unsigned long long)(2 * (uint64_t)h->N), h->N);
