@@ -704,27 +704,31 @@ void place_host(BufferSet &S, void *base, int planes, int per_plane) {
 }
 
 // Control words and records of the last harmonic summing of a set whose stream
-// has completed: from host memory where they are there.
-fdas_status fetch_records(fdas_handle *h, BufferSet &S, unsigned *ctrl, bool records,
-                          std::vector<std::pair<unsigned long long, float>> *out) {
+// has completed: from host memory where they are there (and valid until the set's
+// next search), else from copies in `own_*`.
+struct Records {
+  const unsigned long long *key = nullptr;
+  const float *pwr = nullptr;
+  uint32_t n = 0;
+  std::vector<unsigned long long> own_key;
+  std::vector<float> own_pwr;
+};
+fdas_status fetch_records(fdas_handle *h, BufferSet &S, unsigned *ctrl, bool records, Records *out) {
   if (S.ctrl_valid) std::memcpy(ctrl, S.h_ctrl, sizeof(unsigned) * kCtrlWords);
   else CK(h, cudaMemcpy(ctrl, S.d_ctrl, sizeof(unsigned) * kCtrlWords, cudaMemcpyDeviceToHost));
   if (!records) return FDAS_OK;
   const uint32_t stored = std::min(ctrl[kCtrlTotal], (unsigned)h->cap);
-  out->resize(stored);
-  const unsigned long long *keys = S.h_key;
-  const float *pwrs = S.h_pwr;
-  std::vector<unsigned long long> kv;
-  std::vector<float> pv;
+  out->n = stored;
+  out->key = S.h_key;
+  out->pwr = S.h_pwr;
   if (stored && !(S.results_on_host && stored <= kHostRec)) {
-    kv.resize(stored);
-    pv.resize(stored);
-    CK(h, cudaMemcpy(kv.data(), S.d_key, sizeof(unsigned long long) * stored, cudaMemcpyDeviceToHost));
-    CK(h, cudaMemcpy(pv.data(), S.d_pwr, sizeof(float) * stored, cudaMemcpyDeviceToHost));
-    keys = kv.data();
-    pwrs = pv.data();
+    out->own_key.resize(stored);
+    out->own_pwr.resize(stored);
+    CK(h, cudaMemcpy(out->own_key.data(), S.d_key, sizeof(unsigned long long) * stored, cudaMemcpyDeviceToHost));
+    CK(h, cudaMemcpy(out->own_pwr.data(), S.d_pwr, sizeof(float) * stored, cudaMemcpyDeviceToHost));
+    out->key = out->own_key.data();
+    out->pwr = out->own_pwr.data();
   }
-  for (uint32_t i = 0; i < stored; ++i) (*out)[i] = {keys[i], pwrs[i]};
   return FDAS_OK;
 }
 
@@ -1341,8 +1345,8 @@ fdas_status fdas_retrieve_candidate_list(fdas_handle *h, fdas_candidate *out, ui
   if (st != FDAS_OK) return st;
   BufferSet &S = h->set[ab];
   unsigned ctrl[kCtrlWords];
-  std::vector<std::pair<unsigned long long, float>> recs;
-  if ((st = fetch_records(h, S, ctrl, capacity > 0, &recs)) != FDAS_OK) return st;
+  Records found;
+  if ((st = fetch_records(h, S, ctrl, capacity > 0, &found)) != FDAS_OK) return st;
   uint32_t total = 0;
   for (int pl = 0; pl < h->P; ++pl) total += ctrl[kCtrlCount + pl];
   const uint32_t stored = std::min(ctrl[kCtrlTotal], (unsigned)h->cap);
@@ -1352,6 +1356,8 @@ fdas_status fdas_retrieve_candidate_list(fdas_handle *h, fdas_candidate *out, ui
     return FDAS_OK;
   }
   // (harmonic, template, bin) order, as hsum.py lists its detections
+  std::vector<std::pair<unsigned long long, float>> recs(stored);
+  for (uint32_t i = 0; i < stored; ++i) recs[i] = {found.key[i], found.pwr[i]};
   std::sort(recs.begin(), recs.end(), [](const auto &a, const auto &b) { return a.first < b.first; });
   const uint32_t n = std::min(stored, capacity);
   for (uint32_t i = 0; i < n; ++i) {
@@ -1379,9 +1385,8 @@ fdas_status fdas_retrieve_candidates_ring(fdas_handle *h, uint32_t *detection_lo
   if (st != FDAS_OK) return st;
   BufferSet &S = h->set[ab];
   unsigned ctrl[kCtrlWords];
-  std::vector<std::pair<unsigned long long, float>> recs;
+  Records recs;
   if ((st = fetch_records(h, S, ctrl, true, &recs)) != FDAS_OK) return st;
-  const uint32_t stored = (uint32_t)recs.size();
   // FPGA geometry of the shipped design: groups of 4 templates, bundles of 2
   // bins, 64 slots of 8 lanes per plane (gen_info.h:47-54)
   constexpr int kGroup = 4, kBundle = 2, kSlots = 64, kLanes = 8;
@@ -1398,10 +1403,10 @@ fdas_status fdas_retrieve_candidates_ring(fdas_handle *h, uint32_t *detection_lo
     float pwr;
   };
   std::vector<std::vector<Hit>> per_plane(h->P);
-  for (uint32_t i = 0; i < stored; ++i) {
-    const int plane = (int)(recs[i].first >> 48);
-    const int row = (int)((recs[i].first >> 32) & 0xffffu);
-    const uint32_t bin = (uint32_t)(recs[i].first & 0xffffffffu);
+  for (uint32_t i = 0; i < recs.n; ++i) {
+    const int plane = (int)(recs.key[i] >> 48);
+    const int row = (int)((recs.key[i] >> 32) & 0xffffu);
+    const uint32_t bin = (uint32_t)(recs.key[i] & 0xffffffffu);
     const int t = row - h->H;
     if ((which == FDAS_NEGATIVE_ACCELERATIONS && t > 0) || (which == FDAS_POSITIVE_ACCELERATIONS && t < 0)) continue;
     const int at = t < 0 ? -t : t;
@@ -1409,7 +1414,7 @@ fdas_status fdas_retrieve_candidates_ring(fdas_handle *h, uint32_t *detection_lo
     x.ev = ((unsigned long long)(at / kGroup) << 32) | (bin / kBundle);
     x.lane = (at % kGroup) * kBundle + (int)(bin % kBundle);
     x.loc = (((unsigned)plane & 7u) << 29) | (((unsigned)row & 0x7fu) << 22) | (bin & 0x3fffffu);
-    x.pwr = recs[i].second;
+    x.pwr = recs.pwr[i];
     per_plane[plane].push_back(x);
   }
   for (int pl = 0; pl < h->P; ++pl) {
