@@ -41,11 +41,11 @@ constexpr int kCtrlBound = kCtrlItems + 1;           // + plane: boundary record
 constexpr int kCtrlWords = kCtrlBound + kMaxPlanes;   // zeroed before every harmonic summing
 constexpr int kCtrlFtcStatus = kCtrlWords;           // FT-convolution status, zeroed before each FT convolution
 constexpr int kCtrlTileStatus = kCtrlWords + 1;      // tiling status (tensor-core form), zeroed before each tiling
-// three 64-bit times: end of FT convolution (the latest CTA's), tiling, search
+// two 64-bit times: end of FT convolution (the latest CTA's), tiling
 constexpr int kCtrlStamp = (kCtrlWords + 3) & ~1;
 constexpr int kCtrlZeroed = kCtrlStamp + 2;          // words a search starts from zero
-constexpr int kEndFtc = 0, kEndTiling = 1, kEndSearch = 2;
-constexpr int kCtrlStride = kCtrlStamp + 6;          // control words per buffer set
+constexpr int kEndFtc = 0, kEndTiling = 1;
+constexpr int kCtrlStride = kCtrlStamp + 4;          // control words per buffer set
 constexpr uint32_t kDefaultCapacity = 1u << 22;     // candidate records per buffer set
 constexpr uint32_t kMaxCapacity = 1u << 27;
 constexpr int kRecheckCap = 65536;
@@ -71,6 +71,7 @@ struct BufferSet {
   float *h_cpwr = nullptr;
   unsigned long long *h_key = nullptr;
   float *h_pwr = nullptr;
+  unsigned long long *h_end = nullptr;  // end times of the CTAs of the last kernel
   bool results_on_host = false;  // the last harmonic summing was enqueued whole: they are the device's
   uint4 *d_rc = nullptr;
   unsigned *d_hist = nullptr;
@@ -546,8 +547,8 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
   f.status = p.status;
   f.ctrl = S.d_ctrl;
   f.host_ctrl = S.h_ctrl;
-  f.n_ctrl = kCtrlStamp + 4;
-  f.stamp = chain ? reinterpret_cast<unsigned long long *>(S.h_ctrl + kCtrlStamp) + kEndSearch : nullptr;
+  f.n_ctrl = kCtrlStride;
+  f.stamp = chain ? S.h_end : nullptr;
   // Host memory written by the kernels saves each retrieval its copies (four from
   // pageable memory: 55 us for 442 records before, 20 after)
   f.host_loc = S.h_cloc;
@@ -673,28 +674,32 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
 // the end of the one before, so that a wait (for the other set's kernels) counts
 // for the stage that waited.  In a chain the tiling gets what the events around it
 // leave beside the kernels' end times.
-void stage_times(const BufferSet &S, float *ms3) {
+void stage_times(const BufferSet &S, int planes, float *ms3) {
   if (!S.stamped) {
     const int at[4] = {S.ev_in, 2, 3, S.ev_hs};
     for (int i = 0; i < 3; ++i) ms3[i] = elapsed(S.ev[at[i]], S.ev[at[i + 1]]);
     return;
   }
-  unsigned long long t[3];
+  unsigned long long t[2], end = 0;
   std::memcpy(t, S.h_ctrl + kCtrlStamp, sizeof(t));
+  for (int i = 0; i < planes * kFinSlices; ++i) end = std::max(end, S.h_end[i]);
   ms3[1] = std::max(0.f, (float)(1e-6 * (double)(long long)(t[kEndFtc] - t[kEndTiling])));
-  ms3[2] = std::max(0.f, (float)(1e-6 * (double)(long long)(t[kEndSearch] - t[kEndFtc])));
+  ms3[2] = std::max(0.f, (float)(1e-6 * (double)(long long)(end - t[kEndFtc])));
   ms3[0] = std::max(0.f, elapsed(S.ev[S.ev_in], S.ev[S.ev_hs]) - ms3[1] - ms3[2]);
 }
 
 // Layout of a set's host memory from `base` (host_bytes() bytes, 16-byte aligned)
 size_t host_bytes(int planes, int per_plane) {
   return ((sizeof(unsigned) * kCtrlStride + 15) & ~size_t(15)) + (sizeof(unsigned long long) + sizeof(float)) * kHostRec +
+         sizeof(unsigned long long) * kMaxPlanes * kFinSlices +
          (((sizeof(uint32_t) + sizeof(float)) * (size_t)planes * per_plane + 15) & ~size_t(15));
 }
 void place_host(BufferSet &S, void *base, int planes, int per_plane) {
   char *p = static_cast<char *>(base);
   S.h_ctrl = reinterpret_cast<unsigned *>(p);
   p += (sizeof(unsigned) * kCtrlStride + 15) & ~size_t(15);
+  S.h_end = reinterpret_cast<unsigned long long *>(p);
+  p += sizeof(unsigned long long) * kMaxPlanes * kFinSlices;
   S.h_key = reinterpret_cast<unsigned long long *>(p);
   p += sizeof(unsigned long long) * kHostRec;
   S.h_pwr = reinterpret_cast<float *>(p);
@@ -917,6 +922,7 @@ fdas_status fdas_initialise_accelerator(const fdas_config *cfg_in, fdas_handle *
     }
     place_host(S, S.h_ctrl, h->P, h->per_plane);
     std::memset(S.h_ctrl, 0, sizeof(unsigned) * kCtrlStride);
+    std::memset(S.h_end, 0, sizeof(unsigned long long) * kMaxPlanes * kFinSlices);
     if (make_hsum_maps(h, S) != FDAS_OK) return bail(FDAS_ERR_CUDA);
     for (auto &ev : S.ev) {
       if ((e = cudaEventCreate(&ev)) != cudaSuccess) {
@@ -1444,7 +1450,7 @@ fdas_status fdas_get_stage_times(fdas_handle *h, fdas_buffer_set ab, float *ms6)
   CK(h, cudaSetDevice(h->cfg.device));
   CK(h, cudaEventSynchronize(S.ev[5]));
   float st[3];
-  stage_times(S, st);
+  stage_times(S, h->P, st);
   ms6[0] = elapsed(S.ev[0], S.ev[S.ev_in]);
   ms6[1] = st[0];
   ms6[2] = st[1];
@@ -1495,7 +1501,7 @@ void fdas_print_stats(fdas_handle *h, fdas_buffer_set ab, int reset) {
   logf(h, "[INFO] Launch  #%u%c complete @ %.3f ms II ~ %.3f ms", h->pipeline_launches, set_c, acc * 1e-6,
        (acc - h->pipeline_accum_ns) * 1e-6);
   float st[3];
-  stage_times(S, st);
+  stage_times(S, h->P, st);
   logf(h, "[INFO]   Preparation duration: %.3f ms", st[0]);
   logf(h, "[INFO]   FT convolution and IFFT duration: %.3f ms", st[1]);
   logf(h, "[INFO]   Harmonic summing duration: %.3f ms", st[2]);
@@ -1519,7 +1525,7 @@ void fdas_print_events(fdas_handle *h, fdas_buffer_set ab) {
     if (!S.stamped || (i != 2 && i != 3)) t[i] = event_ns(h, S.ev[at[i]]);
   if (S.stamped) {
     float st[3];
-    stage_times(S, st);
+    stage_times(S, h->P, st);
     t[3] = std::max(t[1], t[4] - (long long)llround(1e6 * (double)st[2]));
     t[2] = std::max(t[1], t[3] - (long long)llround(1e6 * (double)st[1]));
   }

@@ -16,6 +16,7 @@ constexpr int kMaxPlanes = 16;       // harmonic planes supported by the kernels
 constexpr int kSortCap = 8192;       // boundary records one CTA ranks in shared memory
 constexpr int kMaxCompat = 2048;     // entries per plane of the fixed-size list
 constexpr int kSelBuckets = 2048;    // power buckets of the top-K selection (float bits 30..20)
+constexpr int kFinSlices = 8;        // CTAs per plane that write the fixed-size list (slices of its entries)
 
 // device status bits (per buffer set)
 constexpr int kStatusHsumTimeout = 1;
@@ -57,7 +58,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 __device__ __forceinline__ void stamp_last_block(unsigned long long *at) {
-  if (at && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && threadIdx.x == 0) *at = global_ns();
+  if (at && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *at = global_ns();
 }
 __device__ __forceinline__ void stamp_latest(unsigned long long *at) {
   if (at && threadIdx.x == 0) atomicMax(at, global_ns());
@@ -271,7 +272,7 @@ struct SelectParams {
   const unsigned *ctrl;   // n_ctrl control words, copied to pinned host memory at the end
   unsigned *host_ctrl;
   int n_ctrl;
-  unsigned long long *stamp;  // end time, in pinned host memory
+  unsigned long long *stamp;  // [plane][kFinSlices] end times of the last kernel's CTAs, in pinned host memory
 };
 
 // ---- template spectra / taps in FP64

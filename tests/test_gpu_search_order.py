@@ -105,3 +105,25 @@ def test_first_launch_on_the_second_set(order):
         first, second = (events(p, log, ab) for ab in order)
         p.close()
     assert second["ftc_end"] - first["hsum_end"] >= 0.8 * (lone["ftc_end"] - lone["ftc_begin"])
+
+
+@pytest.mark.parametrize("quantile", [1e-7, 1e-4, 1e-2])
+def test_stages_of_searches_with_many_hits(quantile):
+    """Tiling and FT convolution take what they take, however long the selection of
+    the hits does."""
+    log = io.StringIO()
+    n = 1 << 17
+    p = make_pipeline(n, log=log, candidate_capacity=1 << 21)
+    assert p.upload_templates(template_bank(), FDAS.A)
+    nc = p.get_candidate_list_sz()
+    loc, pwr = np.zeros(nc, np.uint32), np.zeros(nc, np.float32)
+    got = {}
+    for q in (1e-7, quantile):
+        times = []
+        for _ in range(9):
+            assert p.launch(noise(3)[:n].copy(), O.chi2_thresholds(q, 8), loc, pwr, FDAS.AllAccelerations, FDAS.A)
+            assert p.wait(FDAS.A)
+            times.append(p.stage_times(FDAS.A))
+        got[q] = np.median(times, axis=0)
+    print(got)
+    assert abs(got[quantile][1] - got[1e-7][1]) < 0.008 and abs(got[quantile][2] - got[1e-7][2]) < 0.008
