@@ -829,6 +829,7 @@ __global__ void __launch_bounds__(512) recheck_kernel(RecheckParams p) {
   __shared__ double cell[kMaxPlanes];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarps = blockDim.x >> 5;
+  grid_release();
   grid_wait();
   const unsigned n = min(*p.rc_count, (unsigned)p.rc_cap);
   for (unsigned e = blockIdx.x; e < n; e += gridDim.x) {
@@ -884,10 +885,6 @@ __global__ void __launch_bounds__(512) recheck_kernel(RecheckParams p) {
     }
     __syncthreads();
   }
-  // Only now: the histogram, which may then start, is one CTA of 1024 threads per SM.
-  // Started beside these CTAs it found room for two on some SMs and for none on others
-  // (2^17 bins x 8 planes, 80 million hits: 1462 us a search, 960 from here)
-  grid_release();
 }
 
 // ------------------------------------------- deterministic top-K per plane
