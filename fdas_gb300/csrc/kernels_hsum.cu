@@ -1176,8 +1176,17 @@ cudaError_t launch_recheck(const RecheckParams &p, cudaStream_t s, bool pdl) {
 
 cudaError_t launch_select(const SelectParams &p, cudaStream_t s, bool pdl) {
   const int n_sm = current_sm_count();
-  const int hsmem = p.n_planes * kSelBuckets * 4;
-  cudaError_t e = launch_sized(select_hist_kernel, dim3(n_sm), dim3(1024), hsmem, s, pdl, p);
+  // More than half of what an SM has, so that it has room for one CTA: these may start
+  // while the recheck's still hold SMs, and with 64 KB for 8 planes there were two on
+  // some SMs and none on others (2^17 bins x 8 planes, 80 million hits: 1419 us a
+  // search against 942; released at the recheck's end instead, they lose the SMs to the
+  // other set's FT convolution: the loop over both sets at 2^21 1960 -> 2007 us; the
+  // 128 KB of 16 planes for all: 1133).
+  constexpr int kOnePerSm = 116 * 1024;
+  static_assert(2 * kOnePerSm > kHsMaxSmem, "one CTA per SM");
+  const int planes_smem = p.n_planes * kSelBuckets * 4;
+  cudaError_t e = launch_sized(select_hist_kernel, dim3(n_sm), dim3(1024),
+                               planes_smem > kOnePerSm ? planes_smem : kOnePerSm, s, pdl, p);
   if (e != cudaSuccess) return e;
   if ((e = launch_kernel(select_gather_kernel, dim3(4 * n_sm), dim3(256), 0, s, pdl, p)) != cudaSuccess) return e;
   const int fsmem = (kSortCap + kMaxCompat) * (8 + 4);
