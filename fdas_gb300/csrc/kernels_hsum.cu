@@ -79,10 +79,11 @@ struct EmitBuf {
 // hardware (they only feed masked cells).  kHsStages stages deep: full / empty
 // mbarriers, every wait bounded by %globaltimer.
 //
-// Planes 2, 4, 8 and 16 read their values with 8- and 4-byte loads at
-// compile-time offsets; for the others the eight bins map onto offsets
-// from two divisions per plane and the four rows onto two staged rows split at
-// a warp-uniform point, handled by a switch.
+// In the bounds planes 2, 4, 8 and 16 read their values with 8- and 4-byte loads at
+// compile-time offsets, the others at offsets from products by 16-bit reciprocals;
+// in the sums of a whole tile the eight bins of a lane map onto offsets from two
+// divisions per plane, and the four rows onto two staged rows split at a
+// warp-uniform point.
 //
 // HP_1 = FOP[t][f], HP_j = HP_{j-1} + FOP[trunc(t/j)][f/j] accumulated in FP32
 // in this order -- hsum.py:95-120 / hms_baseline.cl.mako:55-84 -- so the
@@ -92,8 +93,12 @@ struct EmitBuf {
 // The warps first look at upper bounds of the sums of their lanes' 4 x 4 cell
 // groups only; where no group's bound reaches a plane's band the item is done.
 // A few groups that do are summed one cell per lane (hs_few_groups); for more,
-// the warp sums its whole tile, marks the planes whose band some cell reaches,
-// and recomputes and emits at those (same values, same order).  The exact sums
+// the warp sums its whole tile and emits at the planes that some bound reached
+// (hs_emit_item), which searches with many hits spend their time on: 2^20 bins x 85
+// rows x 8 planes with 0.1 / 0.3 / 1 / 10% of a plane above its threshold take 574 /
+// 1183 / 1460 / 3000 us a stage, against 1399 / 1640 / 1850 / 3450 with up to eight
+// few groups, a reservation per plane and the exact sums once more to mark the planes,
+// and 928 / 1250 / 1650 / 3300 without bounds.  The exact sums
 // of every cell cost 692 instructions per warp and item at about 5.6 clocks
 // each, and so held a stage for longer than its copies take; with the bounds
 // the copies set the pace.  Stage time (noise, with selection) at 2^21 bins x
@@ -135,14 +140,6 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-// maximum of the 32 cells of a tile (3-input max tree)
-__device__ __forceinline__ float max32(const float (&a)[4][8]) {
-  float m[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-    m[k] = fmax3(fmax3(a[k][0], a[k][1], a[k][2]), fmax3(a[k][3], a[k][4], a[k][5]), fmaxf(a[k][6], a[k][7]));
-  return fmax3(m[0], m[1], fmaxf(m[2], m[3]));
-}
 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -175,18 +172,6 @@ __device__ __forceinline__ void add2(float &a0, float &a1, float b0, float b1) {
   asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(b0), "f"(b1));
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(d));
-}
-
-// acc[k][e] += (k < KS ? c0[e] : c1[e]), KS compile time
-template <int KS>
-__device__ __forceinline__ void add_rows(float (&acc)[4][8], const float (&c0)[8], const float (&c1)[8]) {
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int e = 0; e < 8; e += 2) {
-      if (k < KS) add2(acc[k][e], acc[k][e + 1], c0[e], c0[e + 1]);
-      else add2(acc[k][e], acc[k][e + 1], c1[e], c1[e + 1]);
-    }
 }
 
 // Plane 1 of the warp's tile: 4 templates x 8 bins; cells outside the
@@ -340,107 +325,6 @@ __device__ __noinline__ void hs_emit_item(const HsumParams *pp, const float *sta
   hs_emit_item_body<NW>(*pp, stage, eb, f0, sgn, tlo, t0, need);
 }
 
-// The exact sums of the warp's tile: planes (bit j - 1) where a cell of this
-// lane reaches the band.
-template <int MAXP, int NW>
-__device__ __forceinline__ unsigned hs_exact_marks(const HsumParams &p, const float *stage, int f0, int sgn, int tlo,
-                                                   int t0, int lane) {
-  // lane l holds bins f0 + 4 l + {0..3} and f0 + 128 + 4 l + {0..3}: the
-  // lanes of a warp read consecutive 16-byte words (no bank conflicts)
-  const int F = f0 + 4 * lane;
-  float acc[4][8];
-  hs_load_plane1<NW>(acc, stage, p, f0, sgn, tlo, t0, F);
-  // ub: an upper bound of the lane's tile maximum.  Rounded addition is
-  // monotone, so ub + (largest value added) bounds every new sum, and the
-  // exact maximum (a 3-input max tree) is only needed where the bound reaches
-  // a plane's band
-  float ub = max32(acc);
-  unsigned need_lane = ub >= p.trig[0] ? 1u : 0u;  // this lane's marks; one vote per item
-  hs_sfor<MAXP - 1>([&](auto JJ) {
-    constexpr int j = decltype(JJ)::value + 2;
-    if (j <= p.n_planes) {
-      const int a0 = (f0 / j) & ~3;
-      const int bw = p.bw[j], bh = p.bh[j];
-      const float *box = stage + p.soff[j];
-      // f0 is a multiple of 256, so for j = 2, 4, 8, 16 the box starts at f0 / j
-      float vmax;
-      if constexpr (j == 2) {
-        const float *r0 = box + srow(t0 / 2, bh, sgn) * bw + 2 * lane;
-        const float *r1 = r0 + sgn * bw;
-        const float2 a0v = *reinterpret_cast<const float2 *>(r0), b0v = *reinterpret_cast<const float2 *>(r0 + 64);
-        const float2 a1v = *reinterpret_cast<const float2 *>(r1), b1v = *reinterpret_cast<const float2 *>(r1 + 64);
-        vmax = fmax3(fmax3(a0v.x, a0v.y, b0v.x), fmax3(b0v.y, a1v.x, a1v.y), fmaxf(b1v.x, b1v.y));
-  #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const float2 va = kk < 2 ? a0v : a1v, vb = kk < 2 ? b0v : b1v;
-          add2(acc[kk][0], acc[kk][1], va.x, va.x);
-          add2(acc[kk][2], acc[kk][3], va.y, va.y);
-          add2(acc[kk][4], acc[kk][5], vb.x, vb.x);
-          add2(acc[kk][6], acc[kk][7], vb.y, vb.y);
-        }
-      } else if constexpr (hs_one_value(j)) {  // planes 4, 8 and 16: one value per group
-        const float *r0 = box + srow(t0 / j, bh, sgn) * bw + lane / (j / 4);
-        const float va = r0[0], vb = r0[128 / j];
-        vmax = fmaxf(va, vb);
-  #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-  #pragma unroll
-          for (int e = 0; e < 8; e += 2) add2(acc[kk][e], acc[kk][e + 1], e < 4 ? va : vb, e < 4 ? va : vb);
-      } else {
-        const int rb = t0 / j;
-        const int kstar = j - (t0 - rb * j);  // warp-uniform: first k with trunc((t0+k)/j) = rb + 1
-        const float *r0 = box + srow(rb, bh, sgn) * bw - a0;
-        const float *r1 = r0 + sgn * bw;
-        float c0[8], c1[8];
-        // bins F + c and F + 128 + c (c < 4) sit at (F + c) / j = qa + (ra + c >= j)
-        // (ra + 3 < 2 j), and likewise for the second group: two divisions per
-        // plane, and two staged values per group and row, qa and qa + 1
-        // (inside the box)
-        const int qa = F / j, ra = F - qa * j;
-        const int qb = (F + 128) / j, rg = F + 128 - qb * j;
-        bool hi_a[4], hi_b[4];  // cell c takes the value at q + 1
-  #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          hi_a[c] = ra + c >= j;
-          hi_b[c] = rg + c >= j;
-        }
-        const float2 va = make_float2(r0[qa], r0[qa + 1]), vb = make_float2(r0[qb], r0[qb + 1]);
-  #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          c0[c] = hi_a[c] ? va.y : va.x;
-          c0[c + 4] = hi_b[c] ? vb.y : vb.x;
-        }
-        // the bound may include a value no cell takes: still an upper bound
-        vmax = fmaxf(fmaxf(va.x, va.y), fmaxf(vb.x, vb.y));
-        if (kstar < 4) {  // the second row only where the four rows split
-          const float2 wa = make_float2(r1[qa], r1[qa + 1]), wb = make_float2(r1[qb], r1[qb + 1]);
-  #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            c1[c] = hi_a[c] ? wa.y : wa.x;
-            c1[c + 4] = hi_b[c] ? wb.y : wb.x;
-          }
-          vmax = fmax3(vmax, fmaxf(wa.x, wa.y), fmaxf(wb.x, wb.y));
-        } else {
-  #pragma unroll
-          for (int e = 0; e < 8; ++e) c1[e] = 0.f;
-        }
-        switch (kstar < 4 ? kstar : 4) {
-          case 1: add_rows<1>(acc, c0, c1); break;
-          case 2: add_rows<2>(acc, c0, c1); break;
-          case 3: add_rows<3>(acc, c0, c1); break;
-          default: add_rows<4>(acc, c0, c1); break;
-        }
-      }
-      ub += vmax;
-      if (ub >= p.trig[j - 1]) {  // per lane: no vote, no warp-wide branch in the plane loop
-        ub = max32(acc);
-        if (ub >= p.trig[j - 1]) need_lane |= 1u << (j - 1);
-      }
-    }
-  });
-  return need_lane;
-}
-
 // Where a warp's four rows lie in the staged box of plane j: float offset in the
 // stage of the first row trunc(t0 / j) and, in the upper half-word, of the last,
 // trunc((t0 + 3) / j) (the rows in between are one of the two).
@@ -458,7 +342,7 @@ __device__ __forceinline__ unsigned hs_row_offsets(const HsumParams &p, int j, i
 // that every cell's own sums take.
 struct HsBounds {
   float a, b;
-  bool hit_a, hit_b;
+  unsigned hit_a, hit_b;  // planes (bit j - 1) whose band the bound reaches
 };
 __device__ __forceinline__ float fmax4(float4 v) { return fmaxf(fmax3(v.x, v.y, v.z), v.w); }
 __device__ __forceinline__ void hs_bound_plane1(HsBounds &u, const float *stage, unsigned row, float trig, int lane) {
@@ -467,8 +351,8 @@ __device__ __forceinline__ void hs_bound_plane1(HsBounds &u, const float *stage,
   const float4 b0 = r[32], b1 = r[kHsBins / 4 + 32], b2 = r[2 * (kHsBins / 4) + 32], b3 = r[3 * (kHsBins / 4) + 32];
   u.a = fmaxf(fmax3(fmax4(a0), fmax4(a1), fmax4(a2)), fmax4(a3));
   u.b = fmaxf(fmax3(fmax4(b0), fmax4(b1), fmax4(b2)), fmax4(b3));
-  u.hit_a = u.a >= trig;
-  u.hit_b = u.b >= trig;
+  u.hit_a = u.a >= trig ? 1u : 0u;
+  u.hit_b = u.b >= trig ? 1u : 0u;
 }
 // `where`: f0 mod j | (f0 / j - box start) << 8
 template <int j>
@@ -496,19 +380,23 @@ __device__ __forceinline__ void hs_bound_plane(HsBounds &u, const float *stage, 
     u.a += fmaxf(fmax3(s0[qa], s0[ha], s1[qa]), s1[ha]);
     u.b += fmaxf(fmax3(s0[qb], s0[hb], s1[qb]), s1[hb]);
   }
-  u.hit_a |= u.a >= trig;
-  u.hit_b |= u.b >= trig;
+  if (u.a >= trig) u.hit_a |= 1u << (j - 1);
+  if (u.b >= trig) u.hit_b |= 1u << (j - 1);
 }
 
 // The cells of a few 4 x 4 groups (bit l of hit_a / hit_b: lane l's group of
 // the first / second half of the bins), one cell per lane and two groups at a
 // time: their sums, and the hits and near-threshold cells among them.  On noise
 // a warp that does not pass on its bounds has one or two such groups, so this
-// is a fifth of the work of the whole tile's exact sums.
-constexpr int kHsFewGroups = 8;
+// is a fifth of the work of the whole tile's exact sums.  One reservation in the list
+// serves all planes of the two groups (one per plane: 2^17 bins x 85 x 8 with 0.1% of
+// the cells above the threshold 270 us a stage, 244 so).  Up to 16 groups: with eight
+// 0.1 / 0.3% take 895 / 1128 us a stage at 2^20 bins x 85 x 8 against 574 / 1183, and
+// three strong signals the same.
+constexpr int kHsFewGroups = 16;
 template <int MAXP, int NW>
-__device__ __forceinline__ void hs_few_groups_body(const HsumParams &p, const float *stage, EmitBuf *eb, int f0, int sgn,
-                                                   int tlo, int t0, unsigned hit_a, unsigned hit_b) {
+__device__ __forceinline__ void hs_few_groups(const HsumParams &p, const float *stage, EmitBuf *eb, int f0, int sgn,
+                                              int tlo, int t0, unsigned hit_a, unsigned hit_b) {
   const int lane = threadIdx.x & 31;
   unsigned long long todo = (unsigned long long)hit_b << 32 | hit_a;
 #pragma unroll 1
@@ -542,26 +430,35 @@ __device__ __forceinline__ void hs_few_groups_body(const HsumParams &p, const fl
       }
     });
     if (!live) hits = near = 0;
-    if (__any_sync(0xffffffffu, hits | near)) {
-      const int row = p.half + sgn * t, bin = f0 + off;
-      const unsigned below = (1u << lane) - 1u;
+    const int row = p.half + sgn * t, bin = f0 + off;
+    const unsigned below = (1u << lane) - 1u;
+    // one reservation for the hits of all planes, stored plane by plane
+    const unsigned total = __reduce_add_sync(0xffffffffu, (unsigned)__popc(hits));
+    if (total) {
+      unsigned base = 0;
+      if (lane == 0) {
+        base = atomicAdd(p.cand_total, total);
+        if (base + total > (unsigned)p.cand_cap) atomicOr(p.status, kStatusCandidateOverflow);
+      }
+      unsigned at = __shfl_sync(0xffffffffu, base, 0);
       hs_sfor<MAXP>([&](auto JJ) {
         constexpr int i = decltype(JJ)::value;
         if (i < p.n_planes) {
           const unsigned mh = __ballot_sync(0xffffffffu, (hits >> i) & 1u);
-          if (mh) {
-            unsigned base = 0;
-            if (lane == 0) {
-              base = atomicAdd(p.cand_total, (unsigned)__popc(mh));
-              atomicAdd(&eb->pc[i], (unsigned)__popc(mh));
-              if (base + __popc(mh) > (unsigned)p.cand_cap) atomicOr(p.status, kStatusCandidateOverflow);
-            }
-            const unsigned g = __shfl_sync(0xffffffffu, base, 0) + __popc(mh & below);
-            if (((hits >> i) & 1u) && g < (unsigned)p.cand_cap) {
-              p.cand_key[g] = cand_key(i, row, bin);
-              p.cand_pwr[g] = hp[i];
-            }
+          const unsigned g = at + __popc(mh & below);
+          if (((hits >> i) & 1u) && g < (unsigned)p.cand_cap) {
+            p.cand_key[g] = cand_key(i, row, bin);
+            p.cand_pwr[g] = hp[i];
           }
+          if (mh && lane == 0) atomicAdd(&eb->pc[i], (unsigned)__popc(mh));
+          at += __popc(mh);
+        }
+      });
+    }
+    if (__any_sync(0xffffffffu, near)) {
+      hs_sfor<MAXP>([&](auto JJ) {
+        constexpr int i = decltype(JJ)::value;
+        if (i < p.n_planes) {
           const unsigned mn = __ballot_sync(0xffffffffu, (near >> i) & 1u);
           if (mn) {
             unsigned base = 0;
@@ -577,13 +474,6 @@ __device__ __forceinline__ void hs_few_groups_body(const HsumParams &p, const fl
     }
   }
 }
-// (out of line where 16 consumer warps leave 96 registers: the caller's loop would spill)
-template <int MAXP, int NW>
-__device__ __noinline__ void hs_few_groups(const HsumParams *pp, const float *stage, EmitBuf *eb, int f0, int sgn,
-                                           int tlo, int t0, unsigned hit_a, unsigned hit_b) {
-  hs_few_groups_body<MAXP, NW>(*pp, stage, eb, f0, sgn, tlo, t0, hit_a, hit_b);
-}
-
 // NW consumer warps cover the rows of a half, 4 each: 16 for banks above 87
 // rows, 11 above 47, else 6, whose stages are half as large so that five fit
 // (2^21 bins x 43 rows x 8 planes 133 us a stage against 155 with 11 warps and
@@ -759,18 +649,14 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
         if (j <= P)
           hs_bound_plane<j>(u, stage, rj[j], at[j], p.trig[j - 1], lane);
       });
-      const unsigned hit_a = __ballot_sync(0xffffffffu, u.hit_a), hit_b = __ballot_sync(0xffffffffu, u.hit_b);
+      const unsigned hit_a = __ballot_sync(0xffffffffu, u.hit_a != 0), hit_b = __ballot_sync(0xffffffffu, u.hit_b != 0);
       if (hit_a | hit_b) {
         if (__popc(hit_a) + __popc(hit_b) <= kHsFewGroups) {
-          if constexpr (NW <= 11) hs_few_groups_body<MAXP, NW>(p, stage, &eb, f0, sgn, tlo, t0, hit_a, hit_b);
-          else hs_few_groups<MAXP, NW>(sp, stage, &eb, f0, sgn, tlo, t0, hit_a, hit_b);
+          hs_few_groups<MAXP, NW>(p, stage, &eb, f0, sgn, tlo, t0, hit_a, hit_b);
         } else {
-          const unsigned need =
-              __reduce_or_sync(0xffffffffu, hs_exact_marks<MAXP, NW>(p, stage, f0, sgn, tlo, t0, lane));
-          if (need) {
-            if constexpr (MINB >= 2) hs_emit_item_body<NW>(p, stage, &eb, f0, sgn, tlo, t0, need);
-            else hs_emit_item<NW>(sp, stage, &eb, f0, sgn, tlo, t0, need);
-          }
+          const unsigned need = __reduce_or_sync(0xffffffffu, u.hit_a | u.hit_b);
+          if constexpr (MINB >= 2) hs_emit_item_body<NW>(p, stage, &eb, f0, sgn, tlo, t0, need);
+          else hs_emit_item<NW>(sp, stage, &eb, f0, sgn, tlo, t0, need);
         }
       }
 

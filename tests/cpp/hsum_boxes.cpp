@@ -16,11 +16,15 @@ int main() {
       for (int lane = 0; lane < 32; ++lane)
         for (int group = 0; group < 256; group += 128) {
           const int start = (f0 / j) & ~3, F = f0 + 4 * lane + group;
-          // first column and how many: as hs_exact_marks reads them
-          int col, n = 2;
+          // first column and how many: as the bounds read them (hs_bound_plane)
+          int col, n;
           if (hs_one_value(j)) col = lane / (j / 4) + group / j, n = 1;
-          else if (hs_aligned(j)) col = 2 * lane + group / 2;
-          else col = F / j - start;
+          else if (j == 2) col = 2 * lane + group / 2, n = 2;
+          else {
+            const unsigned M = 65536u / j + 1, x = f0 % j + 4 * lane + group;
+            col = (int)((x * M) >> 16) + ((f0 / j) & 3);
+            n = (int)(((x + 3) * M) >> 16) + ((f0 / j) & 3) - col + 1;
+          }
           last = std::max(last, col + n - 1);
           for (int c = 0; c < 4; ++c) {
             const int want = (F + c) / j - start;
