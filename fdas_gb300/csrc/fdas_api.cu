@@ -492,6 +492,7 @@ fdas_status enqueue_hsum(fdas_handle *h, int ab, const float *thr_in, fdas_fop_p
     return fail(h, FDAS_ERR_UNSUPPORTED, "harmonic summing staging exceeds shared memory (too many templates x planes)");
   S.ctrl_valid = S.results_on_host = false;  // until the kernels that write them are enqueued
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl, 0, sizeof(unsigned) * kCtrlWords, S.stream));
+  if (chain) p.stamp = stamp_at(S, kEndFtc);
   CK(h, launch_hsum(p, S.maps, S.stream, chain));
   // (the batched form's per-trial views have none; with one set in use it is left to the
   // first launch on the other set, which waits for it; in a capture the event would be

@@ -63,6 +63,10 @@ __device__ __forceinline__ void stamp_last_block(unsigned long long *at) {
 __device__ __forceinline__ void stamp_latest(unsigned long long *at) {
   if (at && threadIdx.x == 0) atomicMax(at, global_ns());
 }
+// for a kernel that writes no end time, by the kernel after it where that starts
+__device__ __forceinline__ void stamp_if_none(unsigned long long *at) {
+  if (at && blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(at, 0ull, global_ns());
+}
 template <typename Kernel, typename... Args>
 cudaError_t launch_kernel(Kernel kern, dim3 grid, dim3 block, int smem, cudaStream_t s, bool pdl, Args... args) {
   cudaLaunchAttribute at{};
@@ -177,6 +181,8 @@ struct FtcParams {
   // to `tiles_out` as complex spectra
   const float2 *input = nullptr;
   float2 *tiles_out = nullptr;
+  // end time (group form: in the pair form, whose registers are at their limit, it cost
+  // 2 % of the pipelined mode)
   unsigned long long *stamp = nullptr;
 };
 
@@ -213,6 +219,7 @@ struct HsumParams {
   int lean;               // 1: fewer stages and registers (shares an SM with the FT convolution)
   int inject_stall = 0;   // test hook: the first stage of every CTA is announced on its barriers
                           // but its copies are not issued, so the consumers' waits run out
+  unsigned long long *stamp = nullptr;  // end time of the FT convolution, where its kernel wrote none
 };
 
 // 2-D tensor maps of the FOP (rows x stride floats), one box shape per plane

@@ -291,7 +291,6 @@ __global__ void __launch_bounds__(256, 1) ftc_kernel(FtcParams p) {
       });
     });
   }
-  stamp_latest(p.stamp);
 }
 
 // ---------------------------------------------------------------------------
@@ -409,7 +408,6 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
     tile = next_tile;
     rr = next_rr;
   }
-  stamp_latest(p.stamp);
 }
 
 // ---------------------------------------------------------------------------

@@ -522,6 +522,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) hsum_kernel(const __grid_
   }
   grid_release();
   grid_wait();
+  stamp_if_none(p.stamp);
   __syncthreads();
 
   if (warp == NW) {

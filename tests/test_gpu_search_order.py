@@ -127,3 +127,17 @@ def test_stages_of_searches_with_many_hits(quantile):
         got[q] = np.median(times, axis=0)
     print(got)
     assert abs(got[quantile][1] - got[1e-7][1]) < 0.008 and abs(got[quantile][2] - got[1e-7][2]) < 0.008
+
+
+def test_stages_of_the_pipelined_mode():
+    """The pair form of the FT convolution, which the pipelined mode takes: its time and
+    harmonic summing's fill the search's."""
+    log, thr = io.StringIO(), O.chi2_thresholds(1e-7, 8)
+    p = handle(log, overlap=True)
+    xs, outs = host_arrays(p, 1)
+    for _ in range(3):
+        launched(p, xs, outs, thr, (FDAS.A,))
+    ms = p.stage_times(FDAS.A)
+    print(ms)
+    assert 0 < ms[1] < 0.5 * ms[2] and 0.05 < ms[3] < ms[2]
+    assert abs(ms[:5].sum() - ms[5]) < 0.005
