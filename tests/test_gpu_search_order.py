@@ -77,18 +77,21 @@ def test_stage_times_of_a_search_that_waits():
     xs, outs = host_arrays(p, 2)
     for _ in range(2):
         launched(p, xs, outs, thr, (FDAS.A, FDAS.B))
-    launched(p, xs[1:], outs[1:], thr, (FDAS.B,))
-    lone = p.stage_times(FDAS.B)
-    launched(p, xs, outs, thr, (FDAS.A, FDAS.B))
-    both = p.stage_times(FDAS.B)
-    print(lone, p.stage_times(FDAS.A), both)
+    lone, both = [], []
+    for _ in range(5):
+        launched(p, xs[1:], outs[1:], thr, (FDAS.B,))
+        lone.append(p.stage_times(FDAS.B))
+        launched(p, xs, outs, thr, (FDAS.A, FDAS.B))
+        both.append(p.stage_times(FDAS.B))
+        assert abs(both[-1][:5].sum() - both[-1][5]) < 0.005
+    last, lone, both = both[-1], np.median(lone, axis=0), np.median(both, axis=0)
+    print(lone, both)
     assert lone[1] < 0.5 * lone[2] and lone[3] > 0  # (tiling is a tenth of the FT convolution)
     assert both[2] > 0.9 * lone[2]
     assert both[3] < 1.25 * lone[3] + 0.01
-    assert abs(both[:5].sum() - both[5]) < 0.005
     at = events(p, log, FDAS.B)
     assert list(at.values()) == sorted(at.values())
-    assert abs(1e-6 * (at["hsum_end"] - at["hsum_begin"]) - both[3]) < 0.001
+    assert abs(1e-6 * (at["hsum_end"] - at["hsum_begin"]) - last[3]) < 0.001
 
 
 @pytest.mark.parametrize("order", [(FDAS.A, FDAS.B), (FDAS.B, FDAS.A)])
@@ -107,37 +110,41 @@ def test_first_launch_on_the_second_set(order):
     assert second["ftc_end"] - first["hsum_end"] >= 0.8 * (lone["ftc_end"] - lone["ftc_begin"])
 
 
-@pytest.mark.parametrize("quantile", [1e-7, 1e-4, 1e-2])
+def queued_times(p, x, thr):
+    """Stage times of a search queued behind others on its set, so that the host's
+    part of a launch is in none of them; the median of five."""
+    times = []
+    for _ in range(5):
+        for _ in range(3):
+            assert p.enqueue_search_device(x.data_ptr(), thr, FDAS.AllAccelerations, FDAS.A), p.last_error
+        assert p.synchronize(FDAS.A)
+        times.append(p.stage_times(FDAS.A))
+    return np.median(times, axis=0)
+
+
+@pytest.mark.parametrize("quantile", [1e-4, 1e-2])
 def test_stages_of_searches_with_many_hits(quantile):
     """Tiling and FT convolution take what they take, however long the selection of
     the hits does."""
-    log = io.StringIO()
-    n = 1 << 17
-    p = make_pipeline(n, log=log, candidate_capacity=1 << 21)
+    import torch
+    p = make_pipeline(N, log=io.StringIO(), candidate_capacity=1 << 24)
     assert p.upload_templates(template_bank(), FDAS.A)
-    nc = p.get_candidate_list_sz()
-    loc, pwr = np.zeros(nc, np.uint32), np.zeros(nc, np.float32)
-    got = {}
-    for q in (1e-7, quantile):
-        times = []
-        for _ in range(9):
-            assert p.launch(noise(3)[:n].copy(), O.chi2_thresholds(q, 8), loc, pwr, FDAS.AllAccelerations, FDAS.A)
-            assert p.wait(FDAS.A)
-            times.append(p.stage_times(FDAS.A))
-        got[q] = np.median(times, axis=0)
-    print(got)
-    assert abs(got[quantile][1] - got[1e-7][1]) < 0.008 and abs(got[quantile][2] - got[1e-7][2]) < 0.008
+    x = torch.from_numpy(noise(3).view(np.float32)).cuda()
+    torch.cuda.synchronize()
+    few, many = (queued_times(p, x, O.chi2_thresholds(q, 8)) for q in (1e-7, quantile))
+    print(few, many)
+    assert many[3] > 1.5 * few[3]
+    assert abs(many[1] - few[1]) < 0.008 and abs(many[2] - few[2]) < 0.1 * few[2]
 
 
 def test_stages_of_the_pipelined_mode():
-    """The pair form of the FT convolution, which the pipelined mode takes: its time and
-    harmonic summing's fill the search's."""
-    log, thr = io.StringIO(), O.chi2_thresholds(1e-7, 8)
-    p = handle(log, overlap=True)
-    xs, outs = host_arrays(p, 1)
-    for _ in range(3):
-        launched(p, xs, outs, thr, (FDAS.A,))
-    ms = p.stage_times(FDAS.A)
+    """The pair form of the FT convolution, which the pipelined mode takes: tiling is a
+    twentieth of it, and the stages fill the search."""
+    import torch
+    p = handle(io.StringIO(), overlap=True)
+    x = torch.from_numpy(noise(1).view(np.float32)).cuda()
+    torch.cuda.synchronize()
+    ms = queued_times(p, x, O.chi2_thresholds(1e-7, 8))
     print(ms)
     assert 0 < ms[1] < 0.5 * ms[2] and 0.05 < ms[3] < ms[2]
     assert abs(ms[:5].sum() - ms[5]) < 0.005
