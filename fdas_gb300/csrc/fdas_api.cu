@@ -429,7 +429,10 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which, bool chain)
     if (other.ev_hsum_recorded) CK(h, cudaStreamWaitEvent(S.stream, other.ev_hsum, 0));
   }
   if (!chain) CK(h, cudaMemsetAsync(S.d_ctrl + kCtrlFtcStatus, 0, sizeof(unsigned), S.stream));
-  if (chain) p.stamp = stamp_at(S, kEndFtc);
+  if (chain) {
+    p.stamp = stamp_at(S, kEndFtc);
+    p.stamp_begin = stamp_at(S, kEndTiling);
+  }
   CK(h, launch_ftc(p, S.stream, chain));
   if (!chain) CK(h, cudaEventRecord(S.ev[3], S.stream));
   S.ev_ftc_recorded = !chain;

@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   fill_twiddle2(twt, p.twiddle);
+  stamp_first_block(p.stamp_begin);
   __syncthreads();
   if (item < n_items && tp == 0) {
     if (p.inject_stall) mbar_arrive_expect_tx(bar, kTile * 8);  // test hook: a copy that never comes
