@@ -408,7 +408,7 @@ fdas_status enqueue_ftc(fdas_handle *h, int ab, fdas_fop_part which, bool chain)
   p.variant = h->cfg.precision == 1 ? 3 : h->cfg.precision == 2 ? 4 : 0;
   if (h->inject & FDAS_INJECT_FTC_STALL) {
     p.inject_stall = 1;
-    p.variant = 2;  // the hook lives in the warp-pair FFT kernel
+    p.variant = 2;  // a form of two warps per item: both have the hook
   }
   S.ctrl_valid = false;  // the host copy of the control words predates this stage
   // A search whose spectrum was copied from host memory starts its FT

@@ -491,7 +491,8 @@ struct TwistedTw {
 };
 
 // (a, b) <- (a + t b, -(a - t b)): the second output is one packed operation
-// from the first, with its sign turned
+// from the first, with its sign turned (the butterfly of six multiply-adds of FFTs for
+// fused multiply-add units; the sign saves a negation here)
 __device__ __forceinline__ void bfly(float2 &a, float2 &b, float2 t) {
   const float2 h = f2_fma(make_float2(t.x, t.x), b, a);
   const float2 p = make_float2(fmaf(-t.y, b.y, h.x), fmaf(t.y, b.x, h.y));

@@ -44,9 +44,9 @@ __host__ __device__ inline unsigned long long cand_key(int plane, int row, int b
 // memory only after grid_wait(); the kernel before lets it start with
 // grid_release() (or by ending).  Both do nothing without the launch attribute.
 // Hides launch latency and prologues, which bound short spectra: the
-// allocation-free FT convolution of 4096 bins 18.5 -> 14.2 us, of 100003 x 43 rows
-// 28.8 -> 22.7, a search of 32768 bins 94.8 -> 83.7 us, and to 68.3 without events
-// between its kernels and copies after them, of 2^21 bins 699 -> 691 -> 678.
+// allocation-free FT convolution of 4096 bins takes 10.2 us with it and 12.3 without,
+// of 100003 x 43 rows 20.5 / 23.6, a search of 32768 bins 53 / 71 us, of 2^21 bins 642 /
+// 673; an event between two kernels costs the same 2 us as a plain launch.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Where a kernel's work ends, by %globaltimer (32 ns steps here), or nothing: written by

@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(256, 2) ftc2_kernel(FtcParams p) {
 // number of tiles.
 // Bound by the shared-memory pipe and the FMA pipe about alike (2^19 bins x 85
 // rows: 67% and 65% busy, math-pipe throttling first among the stalls, 475
-// shared-memory wavefronts per item); the pair form below has 654 and its L1TEX
+// shared-memory wavefronts per item); the pair form above has 654 and its L1TEX
 // pipe 78% busy.  FT convolution at 2^21 / 2^19 / 2^15 bins x 85 rows: 303 / 81 /
 // 11.1 us against 432 / 118 / 19.4 us of the pair form.  The same with 6 pairs and the
 // tile in registers (168 a thread) took 361 us, 4 pairs of two rows each 488 us;
@@ -776,8 +776,8 @@ static int ftc_variant() {
 // 1.95, 2.00, 2.65, 2.70, 3.40, 3.45 us (slope over the rounds at 2^19 bins x 85
 // rows; an odd pair leaves two of the four schedulers a warp short), and the
 // launch as long as the CTA with the most steps.  Eight for long spectra (2^19:
-// 89 us, six 92, four 100); short ones do not fill their last round: 65536 bins
-// x 85 rows 22 us with six against 26 with eight, 2^17 33 against 35.
+// 82 us, six 86, four 95); short ones do not fill their last round: 65536 bins
+// x 85 rows 16 us with six against 19 with eight, 2^17 27 against 29.
 static long long group_steps(int n_tiles, int n_rows, int gt) { return (long long)((n_tiles + gt - 1) / gt) * n_rows; }
 static int group_tiles(int n_tiles, int n_rows, int n_sm) {
   static const int step_ns[kGroupPairs] = {1240, 1300, 1950, 2000, 2650, 2700, 3400, 3450};
@@ -798,7 +798,7 @@ cudaError_t launch_ftc(const FtcParams &p, cudaStream_t s, bool pdl) {
   const int n_sm = current_sm_count();
   if ((p.variant == 3 || p.variant == 4) && !p.trials) return launch_ftc_tc(p, p.variant == 4, s);
   const long long items = (long long)p.n_tiles * p.n_rows;
-  if ((p.variant ? p.variant : ftc_variant()) == 1 && !p.inject_stall) {  // the test hook is the pair form's
+  if ((p.variant ? p.variant : ftc_variant()) == 1 && !p.inject_stall) {  // (no test hook in the one-warp form)
     const int smem = ex_smem_bytes();
     auto kern = p.trials ? ftc_kernel<true> : ftc_kernel<false>;
     cudaError_t e = allow_smem(kern, smem);

@@ -102,9 +102,9 @@ struct EmitBuf {
 // of every cell cost 692 instructions per warp and item at about 5.6 clocks
 // each, and so held a stage for longer than its copies take; with the bounds
 // the copies set the pace.  Stage time (noise, with selection) at 2^21 bins x
-// 85 rows x 8 planes, 2^20 x 85 x 16, 300007 x 43 x 16, 2^15 x 85 x 8: 189 /
-// 166 / 70 / 30 us against 238 / 297 / 113 / 40; three strong signals at 2^21:
-// 253 against 292.
+// 85 rows x 8 planes, 2^20 x 85 x 16, 300007 x 43 x 16, 2^15 x 85 x 8: 141 /
+// 110 / 37 / 12 us against 238 / 297 / 113 / 40 before the bounds, the block order below
+// and the dependent launches; three strong signals at 2^21: 240 against 292.
 constexpr int kHsHeader = 1536;  // bytes before the stages: barriers, parameters, items
 struct HsItem {
   int f0, sgn, tlo;
@@ -115,8 +115,8 @@ __device__ __forceinline__ HsItem hs_item(const HsumParams &p, int it) {
   // order with o trailing one bits run down from the top of the lowest
   // nb / 2^o blocks, so blocks b, b / 2, b / 4, ... are staged at about the
   // same time and the sub-harmonic boxes of planes 2, 4, 8 (and 6 with 3) find
-  // the lower blocks in L2: at 2^21 bins 171 us a stage on noise and 244 with
-  // three strong signals, against 189 and 255 from the highest block down.
+  // the lower blocks in L2: at 2^21 bins 141 us a stage on noise and 240 with
+  // three strong signals, against 160 and 255 from the highest block down.
   // Each octave starts with its highest blocks: a signal's harmonic images
   // cover wider bin ranges at higher bins (plane j sums f/k for k <= j), so the
   // items that emit most are handed out early and light ones end the launch.
@@ -711,7 +711,8 @@ __device__ __forceinline__ void df_add_prod(float &s, float &t, float a, float b
 // (8 warps took two turns: harmonic-summing stage of 2^20 bins x 16 planes 134.3 ->
 // 129.5 us, of 300007 bins x 43 rows 52.0 -> 51.1).  Up to 8 planes half of those
 // would be idle, and an SM holds three CTAs of 8 warps but one of 16: 413 entries
-// (2^21 bins, three strong signals) 9.0 against 14.6 us.
+// (2^21 bins, three strong signals) 10.6 against 14.6 us.  (32 warps per SM are launched,
+// four CTAs of 8 or two of 16: what is not resident at once follows as others end.)
 __global__ void __launch_bounds__(512) recheck_kernel(RecheckParams p) {
   __shared__ double cell[kMaxPlanes];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

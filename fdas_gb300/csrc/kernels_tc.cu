@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) ftc_tc_kernel(FtcParams p) {
         for (int jj = 0; jj < 32; ++jj) y[32 * c + jj] += cm[jj];
       }
       const float *yr = y, *yi = y + 32;
-      if (FWD && it < n_items) {  // the tile's spectrum, natural order, unnormalised like fft2048_core
+      if (FWD && it < n_items) {  // the tile's spectrum, natural order, unnormalised like tile_fft_kernel
         float2 *out = p.tiles_out + (long long)it * kTile + n1;
         const float fs = pow2f(6 - sigma);
 #pragma unroll

@@ -293,7 +293,10 @@ fdas_status fdas_set_fault_injection(fdas_handle *h, uint32_t flags);
 
 /* Stage times of the last completed launch on `ab`, in milliseconds:
  * [0] input copy, [1] tiling, [2] FT convolution, [3] harmonic summing,
- * [4] candidate download, [5] total; [0] and [4] are 0 where nothing is copied. */
+ * [4] candidate download, [5] total; [0] and [4] are 0 where nothing is copied.
+ * A stage counts from the end of the one before it, so a wait for the other
+ * set's kernels counts for the stage that waited; launch latencies (a few
+ * microseconds) are the tiling's. */
 fdas_status fdas_get_stage_times(fdas_handle *h, fdas_buffer_set ab, float *ms6);
 
 /* FDAS::get_*_sz (FDAS.h:79-89, FDAS.cpp:688-711) -- element counts. */
